@@ -330,6 +330,34 @@ int qd_pcg_solve_static(int32_t n, int nrhs, const int32_t *d_rowptr, const int3
 int qd_csr_spmv(int32_t n, int nrhs, const int32_t *d_rowptr, const int32_t *d_col,
                 const double *d_A, const double *d_X, double *d_Y, double alpha, void *stream);
 
+/* ---------------------------------------------------------------------------
+ * Poisson step on a structured rectangle of nx x ny cells (P1, nodes row-major,
+ * n = (nx + 1)(ny + 1)): K phi = alpha M rho with phi = h_left[c] on x = 0 and
+ * h_right[c] on x = Lx for right-hand side c, natural elsewhere; FP64 conjugate
+ * gradients preconditioned by a separable solver (cosine transform along y,
+ * tridiagonal solves along x).  Replaces PoissonSolver::solve
+ * (backend/src/poisson.cpp:320-334) and poisson_solver.pyx:238-247.
+ *   plan         from qd_poisson_lattice_plan, 16-byte aligned device memory of
+ *                qd_poisson_lattice_plan_size bytes: d_gx[nx] (d_gy[nx + 1]) is the
+ *                sum over the x-edges between columns i and i + 1 (the y-edges of
+ *                column i) of the edges' conductances -K_ab, over ny; all > 0
+ *   d_K, d_M     FP64 values on one CSR pattern; d_rho, d_X [n][nrhs] row-major
+ *   d_X0         start [n][nrhs] (not d_X; its values on x = 0, Lx are not
+ *                read) or NULL
+ *   tol          as in qd_pcg_solve; h_iters the iterations run
+ * Limits: nx <= 8000, nrhs <= 256.  The call waits for the result.
+ * ------------------------------------------------------------------------- */
+int qd_poisson_lattice_plan_size(int nx, int ny, size_t *bytes);
+int qd_poisson_lattice_plan(int nx, int ny, const double *d_gx, const double *d_gy, void *d_plan,
+                            size_t plan_bytes, void *stream);
+int qd_poisson_lattice_workspace_size(int nx, int ny, int nrhs, size_t *bytes);
+int qd_poisson_lattice_solve(int nx, int ny, int nrhs, const int32_t *d_rowptr,
+                             const int32_t *d_col, const double *d_K, const double *d_M,
+                             const double *d_rho, double alpha, const double *h_left,
+                             const double *h_right, const double *d_X0, double *d_X,
+                             const void *d_plan, double tol, int max_iter, int32_t *h_iters,
+                             double *h_relres, void *d_work, size_t work_bytes, void *stream);
+
 /* Open-system (CAP) pencil products: AX = (H + i Himag) X and MX = M X for b
  * complex vectors (1 <= b <= 64), row-major with re/im interleaved,
  * X[row * ldx + c] and AX/MX[row * ldy + c] (leading dimensions in complex

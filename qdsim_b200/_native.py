@@ -60,6 +60,11 @@ SIGNATURES = {
     "qd_pcg_static_scratch_bytes": (_sz, []),
     "qd_pcg_solve_static": (_int, [_i32, _int, _p, _p, _p, _p, _p, _p, _dbl, _int, _p, _p, _p]),
     "qd_csr_spmv": (_int, [_i32, _int, _p, _p, _p, _p, _p, _dbl, _p]),
+    "qd_poisson_lattice_plan_size": (_int, [_int, _int, _p]),
+    "qd_poisson_lattice_plan": (_int, [_int, _int, _p, _p, _p, _sz, _p]),
+    "qd_poisson_lattice_workspace_size": (_int, [_int, _int, _int, _p]),
+    "qd_poisson_lattice_solve": (_int, [_int, _int, _int, _p, _p, _p, _p, _p, _dbl, _p, _p, _p, _p,
+                                        _p, _dbl, _int, _p, _p, _p, _sz, _p]),
     "qd_cap_spmm": (_int, [_i32, _int, _int, _p, _p, _p, _p, _p, _p, _int, _p, _p, _int, _p]),
     "qd_fe_interpolate": (_int, [_int, _i32, _i32, _dbl, _dbl, _int, _i64, _p, _i64, _p, _p,
                                  _p, _p, _p, _p, _int, _p]),

@@ -5,8 +5,10 @@ Same weak form and boundary conditions as
 element, RHS = M (-rho), phi = V_p on x = 0 and V_n on x = Lx, natural
 elsewhere), without its m^2-scale degenerate-area test that skips every
 element of a nanometre mesh (:126).  Assembly uses the warp-per-row kernel
-(c = eps_r, V = 0); the solve is the batched Jacobi-PCG over any number of
-right-hand sides (bias points) sharing the stiffness matrix.
+(c = eps_r, V = 0); the solve is a batched PCG over any number of right-hand
+sides (bias points) sharing the stiffness matrix: preconditioned by the
+lattice's separable solver (``qd_poisson_lattice_solve``) where that is the
+better form, else by the diagonal (``qd_pcg_solve``).
 
 Units: node coordinates in nm, rho in C/m^3, phi in V.
 """
@@ -19,8 +21,44 @@ import torch
 
 from . import _native as N
 from .fem import FEMProblem, stream_ptr
+from .mesh import StructuredMesh
 
 EPS0 = 8.854187817e-12     # qdsim_cython/solvers/poisson_solver.pyx:28
+
+
+#: Largest condition number of the separably preconditioned operator for which
+#: the lattice form is taken.  Its iterations grow with the square root of this
+#: number (about 14 sqrt(kappa) to 1e-12, at five launches each) and not with
+#: the mesh; the diagonal form's grow with the mesh width (about 3 per cell, at
+#: two launches each).
+LATTICE_KAPPA = 64.0
+LATTICE_MAX_NX = 8000       # qd_poisson_lattice_solve's limits
+LATTICE_MAX_RHS = 256
+
+
+def lattice_means(mesh, eps):
+    """Column means of the edge conductances of a P1 structured mesh: ``gx``
+    [nx] over the x-edges between columns i and i + 1, ``gy`` [nx + 1] over the
+    y-edges of column i (both divided by ny), and the condition number bound:
+    the largest over the smallest ratio of an edge's conductance to what the
+    separable operator gives it (mean, halved on the two boundary rows)."""
+    nx, ny = mesh.nx, mesh.ny
+    r = (mesh.Ly / ny) / (mesh.Lx / nx)
+    e = np.asarray(eps, np.float64).reshape(ny, nx, 2)
+    lo, up = e[:, :, 0], e[:, :, 1]          # triangles with the right angle at v00, v11
+    ex = np.zeros((ny + 1, nx))              # conductance of the x-edge (i, i + 1) of row j
+    ex[:-1] += 0.5 * r * lo
+    ex[1:] += 0.5 * r * up
+    ey = np.zeros((ny, nx + 1))
+    ey[:, :-1] += 0.5 / r * lo
+    ey[:, 1:] += 0.5 / r * up
+    gx, gy = ex.sum(0) / ny, ey.sum(0) / ny
+    w = np.ones(ny + 1)
+    w[0] = w[-1] = 0.5
+    inner = ey[:, 1:-1] / gy[1:-1]           # the end columns are Dirichlet
+    q = np.concatenate([(ex / (w[:, None] * gx)).ravel(), inner.ravel()])
+    kappa = float(q.max() / q.min()) if q.min() > 0.0 and np.isfinite(q.max()) else np.inf
+    return gx, gy, kappa
 
 
 class PoissonProblem:
@@ -38,8 +76,29 @@ class PoissonProblem:
         self.right = np.abs(x - mesh.Lx) < 1e-9 * mesh.Lx
         self.d_fixed = torch.from_numpy((self.left | self.right).astype(np.int32)).to(self.device)
         self._ws = None
+        self._plan = self._lattice_plan(eps_r_elem)
         self.last_iters = 0
         self.last_relres = 0.0
+
+    def _lattice_plan(self, eps):
+        """Device plan of the separable preconditioner, or None where the
+        diagonal form is taken (unstructured mesh, eps varying too much along
+        y, a lattice beyond the kernel's limits)."""
+        m = self.mesh
+        if not isinstance(m, StructuredMesh) or m.nx > LATTICE_MAX_NX:
+            return None
+        gx, gy, kappa = lattice_means(m, eps)
+        if not kappa <= LATTICE_KAPPA:
+            return None
+        L = N.lib()
+        nbytes = C.c_size_t()
+        N.check(L.qd_poisson_lattice_plan_size(m.nx, m.ny, C.byref(nbytes)),
+                "qd_poisson_lattice_plan_size")
+        plan = torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
+        g = torch.from_numpy(np.concatenate([gx, gy])).to(self.device)
+        N.check(L.qd_poisson_lattice_plan(m.nx, m.ny, N.ptr(g), N.ptr(g[m.nx:]), N.ptr(plan),
+                                          plan.numel(), stream_ptr()), "qd_poisson_lattice_plan")
+        return plan
 
     def rhs(self, rho):
         """(1e-18/eps0) M (-rho) on the device; rho [N] or [N, nrhs] (C/m^3)."""
@@ -54,6 +113,16 @@ class PoissonProblem:
 
     def solve(self, rho, V_p, V_n, tol=1e-12, max_iter=20000, x0=None):
         """phi (V) at every node, [N] or [N, nrhs] (device tensor)."""
+        n = self.mesh.num_nodes
+        # The cap counts iterations of the diagonal form, which needs about
+        # 3 max(nx, ny): a call capped below any count that could converge is
+        # left with that form, so that it ends at its cap as it always did.
+        if self._plan is not None and max_iter >= 16 * (self.mesh.nx + self.mesh.ny) + 256:
+            r = rho if isinstance(rho, torch.Tensor) else torch.from_numpy(np.asarray(rho, np.float64))
+            r = r.to(self.device, torch.float64).reshape(n, -1).contiguous()
+            if r.shape[1] <= LATTICE_MAX_RHS:
+                return self._solve_lattice(r, V_p, V_n, tol, max_iter, x0)
+            rho = r
         b = self.rhs(rho)
         n, nrhs = b.shape
         vp = torch.as_tensor(np.broadcast_to(np.asarray(V_p, float), (nrhs,)).copy(),
@@ -75,6 +144,30 @@ class PoissonProblem:
                                N.ptr(self.K), N.ptr(b), N.ptr(X), N.ptr(self.d_fixed), float(tol),
                                int(max_iter), C.byref(iters), C.byref(relres), N.ptr(self._ws),
                                self._ws.numel(), stream_ptr()), "qd_pcg_solve")
+        self.last_iters = iters.value
+        self.last_relres = relres.value
+        return X if nrhs > 1 else X[:, 0]
+
+    def _solve_lattice(self, r, V_p, V_n, tol, max_iter, x0):
+        n, nrhs = r.shape
+        m, L = self.mesh, N.lib()
+        vp = np.ascontiguousarray(np.broadcast_to(np.asarray(V_p, float), (nrhs,)))
+        vn = np.ascontiguousarray(np.broadcast_to(np.asarray(V_n, float), (nrhs,)))
+        X = torch.empty_like(r)
+        if x0 is not None:
+            x0 = x0.to(self.device, torch.float64).reshape(n, nrhs).contiguous()
+        nbytes = C.c_size_t()
+        N.check(L.qd_poisson_lattice_workspace_size(m.nx, m.ny, nrhs, C.byref(nbytes)),
+                "qd_poisson_lattice_workspace_size")
+        if self._ws is None or self._ws.numel() < nbytes.value:
+            self._ws = torch.empty(nbytes.value, dtype=torch.uint8, device=self.device)
+        iters = C.c_int32()
+        relres = C.c_double()
+        N.check(L.qd_poisson_lattice_solve(
+            m.nx, m.ny, nrhs, N.ptr(self.fem.d_rowptr), N.ptr(self.fem.d_col), N.ptr(self.K),
+            N.ptr(self.M), N.ptr(r), -1e-18 / EPS0, N.ptr(vp), N.ptr(vn), N.ptr(x0), N.ptr(X),
+            N.ptr(self._plan), float(tol), int(max_iter), C.byref(iters), C.byref(relres),
+            N.ptr(self._ws), self._ws.numel(), stream_ptr()), "qd_poisson_lattice_solve")
         self.last_iters = iters.value
         self.last_relres = relres.value
         return X if nrhs > 1 else X[:, 0]
