@@ -92,7 +92,7 @@ int qd_node_adjacency(int64_t num_nodes, int64_t num_elems, int k, const int32_t
  * host triplet scatter of GPUAccelerator::assemble_matrices
  * (backend/src/gpu_accelerator.cpp:439-642).
  *
- * One warp per CSR row; each row's slots are summed in a fixed order over the
+ * One block per range of CSR rows; each slot is summed in a fixed order over the
  * row's contribution list (deterministic, no atomics).
  *   order        1, 2 or 3 (k = 3, 6, 10 nodes per element)
  *   d_nodes      double[num_nodes*2] (x, y)
@@ -370,6 +370,15 @@ int qd_poisson_lattice_solve(int nx, int ny, int nrhs, const int32_t *d_rowptr,
 int qd_cap_spmm(int32_t n, int b, int vec_fp32, const int32_t *d_rowptr, const int32_t *d_col,
                 const void *d_H, const void *d_Himag, const void *d_M, const void *d_X, int ldx,
                 void *d_AX, void *d_MX, int ldy, void *stream);
+
+/* qd_cap_spmm for rows that are the points of a lattice in row-major order,
+ * `width` rows per line (the rows are taken in tiles, for reuse of the gathered
+ * vectors; the results are the same).  A width that is 0 or does not divide n
+ * is ignored. */
+int qd_cap_spmm_lattice(int32_t n, int32_t width, int b, int vec_fp32, const int32_t *d_rowptr,
+                        const int32_t *d_col, const void *d_H, const void *d_Himag,
+                        const void *d_M, const void *d_X, int ldx, void *d_AX, void *d_MX, int ldy,
+                        void *stream);
 
 /* ---------------------------------------------------------------------------
  * Open-system eigensolve: the k eigenvalues nearest sigma of the complex-

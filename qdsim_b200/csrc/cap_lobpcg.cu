@@ -1210,8 +1210,8 @@ int lobpcg_run(const Problem &P, Work &w, Blocks &bl, int &cur, double tol, int 
   auto AS = [&](int i) { return static_cast<T2 *>(bl.AS[i]); };
   auto MS = [&](int i) { return static_cast<T2 *>(bl.MS[i]); };
   auto spmm = [&](int blk, int c0, int m) {
-    return qd_cap_spmm(n, m, f32 ? 1 : 0, P.rowptr, P.col, H, G, M, S(blk) + c0, ld, AS(blk) + c0,
-                       MS(blk) + c0, ld, s);
+    return qd_cap_spmm_lattice(n, P.prec ? P.prec->nx : 0, m, f32 ? 1 : 0, P.rowptr, P.col, H, G, M,
+                               S(blk) + c0, ld, AS(blk) + c0, MS(blk) + c0, ld, s);
   };
   QD_CUDA_TRY(smem_opt_in<cap_gram_kernel<T>>(size_t(2) * kGStages * kGRows * kGT * sizeof(T2)));
   QD_CUDA_TRY(smem_opt_in<cap_chol_kernel>(kCholSmem));

@@ -1,5 +1,5 @@
 // Host-side CSR pattern, per-row incident-element lists and the slot-sorted
-// contribution plan consumed by the warp-per-row assembly kernel.
+// contribution plan consumed by the assembly kernel.
 //
 // The reference builds triplet lists and lets Eigen / scipy sum duplicates
 // (backend/src/fem.cpp:116-151, qdsim_cython/solvers/schrodinger_solver.pyx:

@@ -1,5 +1,5 @@
 """Finite-element problems on the GPU: CSR pattern (host C++), device-resident
-mesh and coefficient arrays, and the warp-per-row assembly kernel.
+mesh and coefficient arrays, and the row-block assembly kernel.
 
 Units are the library's scaled ones: lengths in nm, energies in eV, kinetic
 coefficient ``c = hbar^2/(2 m*)`` in eV nm^2.  ``C0_EV_NM2`` converts a mass

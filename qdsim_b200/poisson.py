@@ -4,7 +4,7 @@ Same weak form and boundary conditions as
 ``qdsim_cython/solvers/poisson_solver.pyx`` (P1 stiffness with eps_r per
 element, RHS = M (-rho), phi = V_p on x = 0 and V_n on x = Lx, natural
 elsewhere), without its m^2-scale degenerate-area test that skips every
-element of a nanometre mesh (:126).  Assembly uses the warp-per-row kernel
+element of a nanometre mesh (:126).  Assembly uses the row-block kernel
 (c = eps_r, V = 0); the solve is a batched PCG over any number of right-hand
 sides (bias points) sharing the stiffness matrix: preconditioned by the
 lattice's separable solver (``qd_poisson_lattice_solve``) where that is the
