@@ -23,8 +23,8 @@
 //   rr     : per dot (one CTA): convergence test, A = sum_c A_c, B = sum_c B_c,
 //            orthonormal basis (Cholesky dropping dependent P directions, or
 //            SVQB), the B lowest Ritz pairs (tridiagonalisation, bisection,
-//            inverse iteration), Ritz coefficients Y -- all FP64 in shared
-//            memory
+//            inverse iteration), Ritz coefficients Y -- all FP64, in registers
+//            and shared memory
 //   update : X = S Y, P = [W P] Y_wp
 // Recomputing the products of X and P every iteration (instead of updating
 // them with the Ritz coefficients) keeps the residual consistent with X even
@@ -73,6 +73,7 @@ constexpr double kCholPivot32 = 1e-5;    // smallest Cholesky pivot of the scale
 // ... in the mixed form's finishing phase: a basis of condition number below
 // ~1e4 orthonormalised by Cholesky keeps its orthogonality to ~1e-12, well
 // inside the 1e-9 eigenvalue target; worse bases go to SVQB
+// (the plain FP64 form as well: its SVQB kept directions down to 1e-12)
 constexpr double kCholPivotMx = 1e-4;
 #ifndef QD_SVQB_TAU64
 #define QD_SVQB_TAU64 1e-12
@@ -1047,267 +1048,420 @@ __device__ void jacobi_cta(double *A, double *V, int n, int ld, double rel, doub
   __syncthreads();
 }
 
-// The nsel lowest eigenpairs of the symmetric n x n matrix A (shared memory,
-// leading dimension ld; destroyed), by
-//   (1) Householder reduction to tridiagonal form T = H^T A H, the reflector
-//       vectors kept in A's columns below the subdiagonal (3 barriers per
-//       column; 8 lanes per row for the matrix-vector product, the rank-2
-//       update's scalar reduced by every warp for itself);
-//   (2) bisection on Sturm counts of T for all nsel eigenvalues at once, a
-//       group of L = min(32, blockDim / nsel) threads per eigenvalue testing
-//       L points of its interval per round ((L+1)-way multisection);
+// Symmetric matrices of the Rayleigh-Ritz step in registers: thread (ty, tx) of
+// 16 x 16 holds entries (ty + 16 a, tx + 16 b), a, b < TM.  Columns that every
+// thread needs go through shared memory, one barrier apart.
+template <int TM> struct Tile {
+  double v[TM][TM];
+  // entry (ty + 16 a, 16 b + tx) for a b known at run time
+  __device__ __forceinline__ double col(int a, int b) const {
+    double x = v[a][0];
+#pragma unroll
+    for (int q = 1; q < TM; ++q) x = b == q ? v[a][q] : x;
+    return x;
+  }
+  __device__ __forceinline__ double row(int a, int b) const {
+    double x = v[0][b];
+#pragma unroll
+    for (int q = 1; q < TM; ++q) x = a == q ? v[q][b] : x;
+    return x;
+  }
+};
+
+// Cholesky of the scaled Gram matrix Bm (unit diagonal, order mu) carried
+// through the projected matrix: with L D L^T = Bm over the kept columns, A
+// becomes L^-1 A L^-T and N becomes L^-1 (unit lower triangular).  A column from
+// `must` on whose pivot is not above `floor` takes no part (its pivot is
+// recorded as 0); false when an earlier one fails.  One barrier per column:
+// column k of Bm and A and row k of N are published a step ahead.
+// s_pub: 6 * 16 TM doubles; s_piv: 16 TM doubles.
+template <int TM>
+__device__ __forceinline__ bool chol_congruence(Tile<TM> &Bm, Tile<TM> &A, Tile<TM> &N, int mu, int must,
+                                double floor, double *s_pub, double *s_piv) {
+  constexpr int S = 16 * TM;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  auto publish = [&](int k) {
+    double *pb = s_pub + (k & 1) * 3 * S, *pa = pb + S, *pn = pa + S;
+    const int kb = k >> 4;
+    if (tx == (k & 15)) {
+#pragma unroll
+      for (int a = 0; a < TM; ++a) {
+        pb[ty + 16 * a] = Bm.col(a, kb);
+        pa[ty + 16 * a] = A.col(a, kb);
+      }
+    }
+    if (ty == (k & 15)) {
+#pragma unroll
+      for (int b = 0; b < TM; ++b) pn[tx + 16 * b] = N.row(kb, b);
+    }
+  };
+  publish(0);
+  for (int k = 0; k < mu; ++k) {
+    __syncthreads();
+    const double *pb = s_pub + (k & 1) * 3 * S, *pa = pb + S, *pn = pa + S;
+    const double piv = pb[k];                  // every thread reads the same value
+    const bool keep = piv > floor;
+    if (!keep && k < must) {
+      __syncthreads();
+      return false;
+    }
+    if (threadIdx.x == 0) s_piv[k] = keep ? piv : 0.0;
+    if (keep) {
+      const double ip = 1.0 / piv, akk = pa[k];
+      double fr[TM], ar[TM];
+#pragma unroll
+      for (int a = 0; a < TM; ++a) {
+        const int i = ty + 16 * a;
+        fr[a] = i > k ? pb[i] * ip : 0.0;
+        ar[a] = pa[i];
+      }
+#pragma unroll
+      for (int b = 0; b < TM; ++b) {
+        const int j = tx + 16 * b;
+        const double bk = pb[j], fc = j > k ? bk * ip : 0.0, t = fma(-fc, akk, pa[j]), nk = pn[j];
+#pragma unroll
+        for (int a = 0; a < TM; ++a) {
+          Bm.v[a][b] = fma(-fr[a], bk, Bm.v[a][b]);
+          A.v[a][b] = fma(-fr[a], t, fma(-ar[a], fc, A.v[a][b]));
+          N.v[a][b] = fma(-fr[a], nk, N.v[a][b]);
+        }
+      }
+    }
+    if (k + 1 < mu) publish(k + 1);            // the buffer read a step ago
+  }
+  __syncthreads();
+  return true;
+}
+
+// The nsel lowest eigenpairs of the symmetric n x n matrix in the tile A
+// (destroyed; zero beyond n), by
+//   (1) Householder reduction to tridiagonal form T = H^T A H in registers, two
+//       barriers per column: y = A x and |x|^2 for the column x are formed
+//       before its reflector v = x - alpha e_1 is known (A v = y - alpha A e_1),
+//       so that one exchange serves both; the reflectors go to Vs;
+//   (2) bisection on Sturm counts of T for all nsel eigenvalues at once, L = 16
+//       or 32 lanes per eigenvalue testing L points of its interval per round,
+//       within a warp.  The counts are the sign changes of the leading minors
+//       p_i = (d_i - x) p_{i-1} - e^2 p_{i-2} (J. H. Wilkinson, The Algebraic
+//       Eigenvalue Problem, 5.38), one multiply-add on the chain per row where
+//       the quotient form has a division; T is scaled to norm 1 and the minors
+//       are rescaled every 8 rows, so that they stay in range;
 //   (3) inverse iteration on T - lambda_j I (Gaussian elimination with row
-//       interchanges, two steps from a fixed pseudo-random start), one
-//       thread per eigenvalue, then classical Gram-Schmidt applied twice
-//       over the nsel vectors in ascending order (orthonormal also inside
-//       clusters of close eigenvalues, which inverse iteration alone does
-//       not separate);
-//   (4) back-transformation Z = H Y, 16 lanes per vector.
+//       interchanges, factored once; a back-substitution from a fixed
+//       pseudo-random vector, then one full step), one thread per
+//       eigenvalue, then classical Gram-Schmidt over the nsel vectors in
+//       ascending order, repeated for a vector that was not yet orthogonal to
+//       1e-6 (inside clusters of close eigenvalues, which inverse iteration
+//       alone does not separate);
+//   (4) back-transformation Z = H Y, 16 lanes per vector, in registers.
 // Eigenvalues ascending into ev[0..nsel), eigenvectors into Z's columns
-// 0..nsel-1 (ld).  work: 3 n nsel doubles; sw: 4 ld + blockDim + 3 nsel
-// doubles (shared memory); nsel <= 16, blockDim >= 16 nsel.  The eigenvalues
-// are accurate to a few units of roundoff times ||A||, the vectors
-// orthonormal to roundoff.
-__device__ void tridiag_lowest_cta(double *A, double *Z, int n, int ld, int nsel, double *ev,
-                                   double *work, double *sw) {
+// 0..nsel-1 (ldz).  work: 4 n nsel doubles; Vs: n x 16 TM doubles; sw: 10 * 16 TM
+// doubles; all shared memory.  nsel <= 16, 256 threads.  The eigenvalues are
+// accurate to a few units of roundoff times ||A||, the vectors orthonormal to
+// roundoff.
+template <int TM>
+__device__ __forceinline__ void tridiag_lowest_cta(Tile<TM> &A, double *Z, int ldz, int n, int nsel, double *ev,
+                                   double *work, double *Vs, double *sw) {
+  constexpr int S = 16 * TM;
+  constexpr unsigned ALL = 0xffffffffu;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  double *sd = sw, *se = sw + ld, *sg = sw + 2 * ld, *sp = sw + 3 * ld;
-  double *sx = sw + 4 * ld;            // [nt] per-thread scratch (counts, dots)
-  double *slo = sx + nt, *shi = slo + nsel, *sdt = shi + nsel;   // [nsel] each
-  __shared__ double s_lohi[3];   // Gershgorin bounds, pivot floor
-  __shared__ int s_open[2];   // intervals still open, by round parity
-  // (1) tridiagonalisation
+  const int tx = tid & 15, ty = tid >> 4;
+  double *sd = sw, *se = sw + S, *sg = sw + 2 * S, *ys = sw + 3 * S, *cs = sw + 4 * S,
+         *xs = sw + 5 * S;                     // xs: two buffers
+  double2 *de = reinterpret_cast<double2 *>(sw + 7 * S);   // (d_i, e_{i-1}^2), scaled
+  double *sdt = sw + 9 * S;
+  // (1)
+  auto publish = [&](int k) {                  // column k below the diagonal, and d_k
+    if (tx == (k & 15)) {
+      double *x = xs + (k & 1) * S;
+#pragma unroll
+      for (int a = 0; a < TM; ++a) {
+        const int i = ty + 16 * a;
+        const double v = A.col(a, k >> 4);
+        x[i] = i > k ? v : 0.0;
+        if (i == k) sd[k] = v;
+      }
+    }
+  };
+  publish(0);
+  __syncthreads();
   for (int k = 0; k + 2 < n; ++k) {
-    const int len = n - k - 1;
-    if (warp == 0) {
-      double sig = 0.0;
-      for (int i = lane; i < len; i += 32) {
-        const double x = A[(k + 1 + i) * ld + k];
-        sig += x * x;
-      }
+    const double *x = xs + (k & 1) * S;
+    double y[TM], s2 = 0.0, xr[TM], xc[TM];
 #pragma unroll
-      for (int o = 16; o; o >>= 1) sig += __shfl_xor_sync(0xffffffffu, sig, o);
-      if (lane == 0) {
-        const double x0 = A[(k + 1) * ld + k];
-        if (sig - x0 * x0 <= 1e-300 * fmax(1.0, sig)) {   // column already reduced
-          se[k] = x0;
-          sg[k] = 0.0;
-        } else {
-          const double alpha = -copysign(sqrt(sig), x0);
-          se[k] = alpha;
-          sg[k] = 1.0 / (sig - x0 * alpha);                 // 2 / v^T v
-          A[(k + 1) * ld + k] = x0 - alpha;                 // v = x - alpha e_1
-        }
-      }
+    for (int a = 0; a < TM; ++a) {
+      xr[a] = x[ty + 16 * a];
+      xc[a] = x[tx + 16 * a];
+      y[a] = 0.0;
+    }
+#pragma unroll
+    for (int b = 0; b < TM; ++b) {
+      s2 = fma(xc[b], xc[b], s2);
+#pragma unroll
+      for (int a = 0; a < TM; ++a) y[a] = fma(A.v[a][b], xc[b], y[a]);
+    }
+#pragma unroll
+    for (int o = 8; o; o >>= 1) {
+      s2 += __shfl_xor_sync(ALL, s2, o);
+#pragma unroll
+      for (int a = 0; a < TM; ++a) y[a] += __shfl_xor_sync(ALL, y[a], o);
+    }
+    if (tx == 0) {
+#pragma unroll
+      for (int a = 0; a < TM; ++a) ys[ty + 16 * a] = y[a];
+    }
+    if (tx == ((k + 1) & 15)) {
+#pragma unroll
+      for (int a = 0; a < TM; ++a) cs[ty + 16 * a] = A.col(a, (k + 1) >> 4);
     }
     __syncthreads();
-    const double g = sg[k];
-    if (g == 0.0) continue;                                  // uniform
-    // p = g A_sub v, 8 lanes per row
-    for (int i0 = 0; i0 < len; i0 += nt / 8) {
-      const int i = i0 + tid / 8, sub = tid & 7;
-      double acc = 0.0;
-      if (i < len) {
-        const double *row = A + (k + 1 + i) * ld + (k + 1);
-        for (int j = sub; j < len; j += 8) acc += row[j] * A[(k + 1 + j) * ld + k];
+    const double x0 = x[k + 1];
+    // |x|^2 is the same sum in every thread, and so is this test
+    if (s2 - x0 * x0 <= 1e-300 * fmax(1.0, s2)) {   // column already reduced
+      if (tid == 0) {
+        se[k] = x0;
+        sg[k] = 0.0;
       }
-      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-      if (i < len && sub == 0) sp[i] = g * acc;
-    }
-    __syncthreads();
-    // A_sub -= v q^T + q v^T, q = p - K v, K = g (v^T p) / 2 (each warp sums it)
-    double K = 0.0;
-    for (int j = lane; j < len; j += 32) K += A[(k + 1 + j) * ld + k] * sp[j];
+    } else {
+      double xy = 0.0;                              // x^T y, each warp for itself
+      for (int i = lane; i < n; i += 32) xy = fma(x[i], ys[i], xy);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) K += __shfl_xor_sync(0xffffffffu, K, o);
-    K *= 0.5 * g;
-    for (int e = tid; e < len * len; e += nt) {
-      const int i = e / len, j = e - i * len;
-      const double vi = A[(k + 1 + i) * ld + k], vj = A[(k + 1 + j) * ld + k];
-      A[(k + 1 + i) * ld + (k + 1 + j)] += 2.0 * K * vi * vj - vi * sp[j] - sp[i] * vj;
+      for (int o = 16; o; o >>= 1) xy += __shfl_xor_sync(ALL, xy, o);
+      const double alpha = -copysign(sqrt(s2), x0);
+      const double g = 1.0 / (s2 - x0 * alpha);     // 2 / v^T v
+      const double vp = g * (xy + alpha * (alpha * cs[k + 1] - 2.0 * ys[k + 1]));
+      const double K = 0.5 * g * vp;
+      double vr[TM], wr[TM];
+#pragma unroll
+      for (int a = 0; a < TM; ++a) {
+        const int i = ty + 16 * a;
+        vr[a] = i == k + 1 ? x0 - alpha : xr[a];
+        wr[a] = i > k ? fma(-K, vr[a], g * (ys[i] - alpha * cs[i])) : 0.0;
+      }
+#pragma unroll
+      for (int b = 0; b < TM; ++b) {
+        const int j = tx + 16 * b;
+        const double vc = j == k + 1 ? x0 - alpha : xc[b];
+        const double wc = j > k ? fma(-K, vc, g * (ys[j] - alpha * cs[j])) : 0.0;
+#pragma unroll
+        for (int a = 0; a < TM; ++a) A.v[a][b] = fma(-vr[a], wc, fma(-wr[a], vc, A.v[a][b]));
+      }
+      if (tid < n) Vs[k * S + tid] = tid == k + 1 ? x0 - alpha : x[tid];
+      if (tid == 0) {
+        se[k] = alpha;
+        sg[k] = g;
+      }
     }
+    publish(k + 1);
     __syncthreads();
   }
+  if (tid == 0) se[n - 2] = xs[((n - 2) & 1) * S + n - 1];
+  // d_{n-1} sits at register (q, q), q = (n - 1) / 16
+  if (tx == ((n - 1) & 15) && ty == tx) {
+#pragma unroll
+    for (int q = 0; q < TM; ++q)
+      if (q == (n - 1) >> 4) sd[n - 1] = A.v[q][q];
+  }
+  __syncthreads();
+  // Gershgorin bounds and the scale (a power of two), each warp for itself
+  double lo0 = 1e300, hi0 = -1e300;
+  for (int i = lane; i < n; i += 32) {
+    const double r = (i > 0 ? fabs(se[i - 1]) : 0.0) + (i + 1 < n ? fabs(se[i]) : 0.0);
+    lo0 = fmin(lo0, sd[i] - r);
+    hi0 = fmax(hi0, sd[i] + r);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    lo0 = fmin(lo0, __shfl_xor_sync(ALL, lo0, o));
+    hi0 = fmax(hi0, __shfl_xor_sync(ALL, hi0, o));
+  }
+  const double big = fmax(fmax(fabs(lo0), fabs(hi0)), 1e-280);
+  const int ex = isfinite(big) ? ilogb(big) + 1 : 0;
+  const double up = scalbn(1.0, ex), dn = scalbn(1.0, -ex);
   for (int i = tid; i < n; i += nt) {
-    sd[i] = A[i * ld + i];
-    if (i == n - 2) se[i] = A[(n - 1) * ld + (n - 2)];
-    if (i >= n - 2) sg[i] = 0.0;
+    const double e = i > 0 ? se[i - 1] * dn : 0.0;
+    // a floor of (1e-16)^2 under e^2: an exact zero would end the recurrence
+    // where x meets an eigenvalue of the leading block
+    de[i] = make_double2(sd[i] * dn, fmax(e * e, 1e-32));
   }
   __syncthreads();
-  if (tid == 0) {
-    double lo = 1e300, hi = -1e300, emax = 0.0;
-    for (int i = 0; i < n; ++i) {
-      const double r = (i > 0 ? fabs(se[i - 1]) : 0.0) + (i + 1 < n ? fabs(se[i]) : 0.0);
-      lo = fmin(lo, sd[i] - r);
-      hi = fmax(hi, sd[i] + r);
-      if (i + 1 < n) emax = fmax(emax, se[i] * se[i]);
-    }
-    const double w = hi - lo;
-    s_lohi[0] = lo - 1e-14 * w - 1e-300;
-    s_lohi[1] = hi + 1e-14 * w + 1e-300;
-    s_lohi[2] = 1e-290 * fmax(1.0, emax);
-  }
-  for (int i = tid; i + 1 < n; i += nt) sp[i] = se[i] * se[i];   // e_i^2
-  __syncthreads();
-  // (2) bisection, all eigenvalues at once
-  const double pivmin = s_lohi[2];
-  const int L = min(32, nt / nsel);
-  const int grp = tid / L, lt = tid - grp * L;
-  if (tid < nsel) {
-    slo[tid] = s_lohi[0];
-    shi[tid] = s_lohi[1];
-  }
-  __syncthreads();
-  for (int round = 0; round < 64; ++round) {
-    if (grp < nsel) {
-      const double lo = slo[grp], hi = shi[grp];
-      const double x = lo + double(lt + 1) * ((hi - lo) / double(L + 1));
-      double q = sd[0] - x;
-      int c = q < 0.0;
-      for (int i = 1; i < n; ++i) {
-        if (fabs(q) < pivmin) q = -pivmin;
-        q = (sd[i] - x) - sp[i - 1] / q;
-        c += q < 0.0;
-      }
-      sx[tid] = double(c);
-    }
-    if (round == 0 && tid == 0) s_open[0] = 0;
-    __syncthreads();
-    if (tid == 0) s_open[(round + 1) & 1] = 0;   // last read a round ago
-    if (tid < nsel) {
-      const int j = tid;
-      const double lo = slo[j], hi = shi[j], step = (hi - lo) / double(L + 1);
-      int l = L;
-      for (int t = 0; t < L; ++t)
-        if (sx[j * L + t] >= double(j + 1)) {
-          l = t;
-          break;
+  // (2)
+  {
+    const int L = nsel <= 8 ? 32 : 16, grp = tid / L, lt = tid & (L - 1);
+    const int j = min(grp, nsel - 1), gl = lane & ~(L - 1);
+    double lo = lo0 * dn - 1e-14, hi = hi0 * dn + 1e-14;
+    for (int round = 0; round < 64; ++round) {
+      const double step = (hi - lo) / double(L + 1);
+      const double x = lo + double(lt + 1) * step;
+      double p0 = 1.0, p1 = de[0].x - x;
+      int c = p1 < 0.0;
+      int i = 1;
+      for (; i + 8 <= n; i += 8) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const double2 t = de[i + u];
+          const double p2 = fma(t.x - x, p1, -(t.y * p0));
+          c += (p2 < 0.0) != (p1 < 0.0);
+          p0 = p1;
+          p1 = p2;
         }
-      const double nlo = l > 0 ? lo + double(l) * step : lo;
-      const double nhi = l < L ? lo + double(l + 1) * step : hi;
-      slo[j] = nlo;
-      shi[j] = nhi;
-      if (nhi - nlo > 4.440892098500626e-16 * fmax(fabs(nlo), fabs(nhi)) + 1e-300)
-        atomicAdd(&s_open[round & 1], 1);
+        const double m = fmax(fabs(p0), fabs(p1));
+        const double f = m < 1e-100 ? 1e100 : (m > 1e100 ? 1e-100 : 1.0);
+        p0 *= f;
+        p1 *= f;
+      }
+      for (; i < n; ++i) {
+        const double2 t = de[i];
+        const double p2 = fma(t.x - x, p1, -(t.y * p0));
+        c += (p2 < 0.0) != (p1 < 0.0);
+        p0 = p1;
+        p1 = p2;
+      }
+      const unsigned over = __ballot_sync(ALL, c > j) >> gl & (L == 32 ? ALL : 0xffffu);
+      const int f = over ? __ffs(over) - 1 : L;   // the first point above the eigenvalue
+      const double nlo = f > 0 ? lo + double(f) * step : lo;
+      const double nhi = f < L ? lo + double(f + 1) * step : hi;
+      lo = nlo;
+      hi = nhi;
+      const bool open = hi - lo > fmax(4.440892098500626e-16 * fmax(fabs(lo), fabs(hi)), 1e-17);
+      if (!__any_sync(ALL, open)) break;
     }
-    __syncthreads();
-    if (s_open[round & 1] == 0) break;                        // uniform
+    if (grp < nsel && lt == 0) ev[grp] = 0.5 * (lo + hi);   // scaled
   }
-  if (tid < nsel) ev[tid] = 0.5 * (slo[tid] + shi[tid]);
   __syncthreads();
-  // (3) inverse iteration, one thread per eigenvalue, vector in Z's column j
+  // (3)
   if (tid < nsel) {
-    const int j = tid;
-    double *dg = work + 3 * n * j, *su = dg + n, *su2 = su + n;
-    double tn = 0.0;
-    for (int i = 0; i < n; ++i) tn = fmax(tn, fmax(fabs(sd[i]), i + 1 < n ? fabs(se[i]) : 0.0));
-    const double tiny = 2.220446049250313e-16 * fmax(tn, 1e-300);
-    const double lam = ev[j];
-    for (int i = 0; i < n; ++i)
-      Z[i * ld + j] = double((uint32_t(j + 1) * 2654435761u + uint32_t(i) * 40503u) % 1000u) / 1000.0 + 0.5;
+    const int j = tid, W = nsel;
+    double *di = work, *su = work + n * W, *su2 = work + 2 * n * W, *ml = work + 3 * n * W;
+    const double tiny = 2.220446049250313e-16, lam = ev[j];
+    unsigned long long swapped = 0;
+    double dc = de[0].x - lam, uc = se[0] * dn;
+    for (int i = 0; i + 1 < n; ++i) {
+      const double e = se[i] * dn, dx = de[i + 1].x - lam, ux = i + 2 < n ? se[i + 1] * dn : 0.0;
+      const bool sw_ = fabs(e) > fabs(dc);
+      double piv = sw_ ? e : dc;
+      if (fabs(piv) < tiny) piv = copysign(tiny, piv);
+      const double inv = 1.0 / piv, m = (sw_ ? dc : e) * inv;
+      const double u1 = sw_ ? dx : uc, u2 = sw_ ? ux : 0.0;
+      di[i * W + j] = inv;
+      su[i * W + j] = u1;
+      su2[i * W + j] = u2;
+      ml[i * W + j] = m;
+      swapped |= (unsigned long long)(sw_) << i;
+      dc = fma(-m, u1, sw_ ? uc : dx);
+      uc = sw_ ? -m * u2 : ux;
+    }
+    if (fabs(dc) < tiny) dc = copysign(tiny, dc);
+    di[(n - 1) * W + j] = 1.0 / dc;
+    double scale = 1.0;
     for (int it = 0; it < 2; ++it) {
-      for (int i = 0; i < n; ++i) {
-        dg[i] = sd[i] - lam;
-        su[i] = i + 1 < n ? se[i] : 0.0;
-        su2[i] = 0.0;
-      }
-      for (int i = 0; i + 1 < n; ++i) {
-        const double b = se[i];
-        double *y = Z + j;
-        if (fabs(b) > fabs(dg[i])) {          // interchange rows i and i + 1
-          const double r0 = b, r1 = dg[i + 1], r2 = su[i + 1];
-          const double s0 = dg[i], s1 = su[i];
-          dg[i] = r0;
-          su[i] = r1;
-          su2[i] = r2;
-          const double t = y[i * ld];
-          y[i * ld] = y[(i + 1) * ld];
-          y[(i + 1) * ld] = t;
-          const double mlt = s0 / r0;
-          dg[i + 1] = s1 - mlt * r1;
-          su[i + 1] = -mlt * r2;
-          y[(i + 1) * ld] -= mlt * y[i * ld];
-        } else {
-          const double piv = dg[i] != 0.0 ? dg[i] : tiny;
-          dg[i] = piv;
-          const double mlt = b / piv;
-          dg[i + 1] -= mlt * su[i];
-          y[(i + 1) * ld] -= mlt * y[i * ld];
+      if (it == 1) {
+        double y = Z[j] * scale;
+        for (int i = 0; i + 1 < n; ++i) {
+          double z = Z[(i + 1) * ldz + j] * scale;
+          if (swapped >> i & 1) {
+            const double t = y;
+            y = z;
+            z = t;
+          }
+          Z[i * ldz + j] = y;
+          y = fma(-ml[i * W + j], y, z);
         }
+        Z[(n - 1) * ldz + j] = y;
       }
-      if (dg[n - 1] == 0.0) dg[n - 1] = tiny;
-      double nrm = 0.0;
+      double x1 = 0.0, x2 = 0.0, nrm = 0.0;
       for (int i = n - 1; i >= 0; --i) {
-        double sacc = Z[i * ld + j];
-        if (i + 1 < n) sacc -= su[i] * Z[(i + 1) * ld + j];
-        if (i + 2 < n) sacc -= su2[i] * Z[(i + 2) * ld + j];
-        const double x = sacc / (dg[i] != 0.0 ? dg[i] : tiny);
-        Z[i * ld + j] = x;
-        nrm += x * x;
+        const double b = it == 0 ? double((uint32_t(j + 1) * 2654435761u + uint32_t(i) * 40503u) % 1000u) / 1000.0 + 0.5
+                                 : Z[i * ldz + j];
+        double acc = b;
+        if (i + 1 < n) acc = fma(-su[i * W + j], x1, fma(-su2[i * W + j], x2, acc));
+        const double x = acc * di[i * W + j];
+        Z[i * ldz + j] = x;
+        nrm = fma(x, x, nrm);
+        x2 = x1;
+        x1 = x;
       }
-      const double inv = rsqrt(fmax(nrm, 1e-300));
-      for (int i = 0; i < n; ++i) Z[i * ld + j] *= inv;
+      scale = rsqrt(fmax(nrm, 1e-300));
     }
+    for (int i = 0; i < n; ++i) Z[i * ldz + j] *= scale;
+    ev[j] = lam * up;
   }
   __syncthreads();
-  // classical Gram-Schmidt, twice per vector, in ascending order: warp w
-  // forms the coefficients against vectors i = w, w + 8, ..., all threads
-  // subtract, warp 0 normalises
+  // classical Gram-Schmidt in ascending order: warp w forms the coefficients
+  // against vectors i = w, w + 8, ..., all threads subtract, warp 0 normalises
   for (int j = 1; j < nsel; ++j) {
     for (int pass = 0; pass < 2; ++pass) {
       for (int i = warp; i < j; i += nt / 32) {
         double dt = 0.0;
-        for (int r = lane; r < n; r += 32) dt += Z[r * ld + i] * Z[r * ld + j];
+        for (int r = lane; r < n; r += 32) dt += Z[r * ldz + i] * Z[r * ldz + j];
 #pragma unroll
-        for (int o = 16; o; o >>= 1) dt += __shfl_xor_sync(0xffffffffu, dt, o);
+        for (int o = 16; o; o >>= 1) dt += __shfl_xor_sync(ALL, dt, o);
         if (lane == 0) sdt[i] = dt;
       }
       __syncthreads();
+      double worst = 0.0;
+      for (int i = 0; i < j; ++i) worst = fmax(worst, fabs(sdt[i]));
       for (int r = tid; r < n; r += nt) {
-        double v = Z[r * ld + j];
-        for (int i = 0; i < j; ++i) v -= sdt[i] * Z[r * ld + i];
-        Z[r * ld + j] = v;
+        double v = Z[r * ldz + j];
+        for (int i = 0; i < j; ++i) v -= sdt[i] * Z[r * ldz + i];
+        Z[r * ldz + j] = v;
       }
       __syncthreads();
+      if (worst <= 1e-6) break;                    // the same in every thread
     }
     if (warp == 0) {
       double nr = 0.0;
-      for (int r = lane; r < n; r += 32) nr += Z[r * ld + j] * Z[r * ld + j];
+      for (int r = lane; r < n; r += 32) nr += Z[r * ldz + j] * Z[r * ldz + j];
 #pragma unroll
-      for (int o = 16; o; o >>= 1) nr += __shfl_xor_sync(0xffffffffu, nr, o);
+      for (int o = 16; o; o >>= 1) nr += __shfl_xor_sync(ALL, nr, o);
       const double inv = rsqrt(fmax(nr, 1e-300));
-      for (int r = lane; r < n; r += 32) Z[r * ld + j] *= inv;
+      for (int r = lane; r < n; r += 32) Z[r * ldz + j] *= inv;
     }
     __syncthreads();
   }
-  // (4) Z = H Y: reflectors applied last first, 16 lanes per vector
+  // (4) Z = H Y: reflectors applied last first
   {
-    const int c = tid >> 4, l16 = tid & 15;
-    const bool live = c < nsel;
+    const int c = min(ty, nsel - 1);
+    double z[TM];
+#pragma unroll
+    for (int a = 0; a < TM; ++a) z[a] = tx + 16 * a < n ? Z[(tx + 16 * a) * ldz + c] : 0.0;
     for (int k = n - 3; k >= 0; --k) {
       const double g = sg[k];
       if (g == 0.0) continue;                                // uniform
-      double dt = 0.0;
-      if (live)
-        for (int r = k + 1 + l16; r < n; r += 16) dt += A[r * ld + k] * Z[r * ld + c];
+      double v[TM], dt = 0.0;
 #pragma unroll
-      for (int o = 8; o; o >>= 1) dt += __shfl_xor_sync(0xffffffffu, dt, o);
+      for (int a = 0; a < TM; ++a) {
+        v[a] = tx + 16 * a < n ? Vs[k * S + tx + 16 * a] : 0.0;
+        dt = fma(v[a], z[a], dt);
+      }
+#pragma unroll
+      for (int o = 8; o; o >>= 1) dt += __shfl_xor_sync(ALL, dt, o);
       dt *= g;
-      if (live)
-        for (int r = k + 1 + l16; r < n; r += 16) Z[r * ld + c] -= dt * A[r * ld + k];
-      __syncwarp();
+#pragma unroll
+      for (int a = 0; a < TM; ++a) z[a] = fma(-dt, v[a], z[a]);
+    }
+    __syncthreads();
+    if (ty < nsel) {
+#pragma unroll
+      for (int a = 0; a < TM; ++a)
+        if (tx + 16 * a < n) Z[(tx + 16 * a) * ldz + ty] = z[a];
     }
   }
   __syncthreads();
 }
 
-// Rayleigh-Ritz on span[X W P] by SVQB: with D the diagonal scaling of the
-// basis Gram B, eigendecompose D B D = U S U^T, drop directions with
-// S < tau max(S) (near-dependent or null columns, e.g. a preconditioned
-// residual that is almost parallel to X), Q = U_keep S_keep^-1/2, then solve
-// the standard problem (Q^T D A D Q) z = theta z and return Y = D Q Z.
+// Rayleigh-Ritz on span[X W P]: with D the diagonal scaling of the basis Gram B,
+// an orthonormal basis Q of the scaled Gram D B D (chol_congruence, or SVQB:
+// eigendecompose D B D = U S U^T, drop directions with S < tau max(S), e.g. a
+// preconditioned residual that is almost parallel to X, Q = U_keep S_keep^-1/2),
+// the B lowest eigenpairs of (Q^T D A D Q) z = theta z, and Y = D Q Z.
+// One CTA per dot, so its latency adds to every iteration: it is bound by the
+// chains of small dependent steps and the barriers between them (about seven
+// cycles per instruction and warp).  With the matrices in registers, the
+// congruence in place of two triangular products, and bisection without
+// divisions it takes about 165 us at B = 16 and 130 us at B = 12 where the form
+// in shared memory took 377 and 220 us (and 500 us with SVQB in every step of the
+// plain FP64 form, which now takes it only when a pivot is small).
 template <int B>
 __global__ void __launch_bounds__(256)
 rr_kernel(DotState *st, const double *partial, const double *norms, double *theta,
@@ -1317,11 +1471,11 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
   double *sA = sm;             // m*m
   double *sB = sA + m * m;     // m*m
   double *sT = sB + m * m;     // m*m
-  double *sZ = sT + m * m;     // m*m
-  double *sD = sZ + m * m;     // m    column scaling
-  double *sE = sD + m;         // m    eigenvalues
+  double *sZ = sT + m * m;     // m*S  (S = m rounded up to 16)
+  double *sD = sZ + m * ((m + 15) / 16 * 16);   // S  column scaling
+  double *sE = sD + (m + 15) / 16 * 16;         // S  pivots, eigenvalues
   double *sR = sE + m;         // B    relative residuals
-  double *sW = sR + B;         // 4m + 256 + 3B  scratch of the tridiagonal eigensolver
+  double *sW = sR + B;         // 10 * 16 TM  scratch of the Cholesky and tridiagonal steps
   __shared__ int s_flag, s_r, s_keep[kMaxM], s_sel[kMaxM];
   __shared__ double s_red[256];
   __shared__ double s_c[kMaxM / 2 + 1], s_s[kMaxM / 2 + 1];
@@ -1418,104 +1572,89 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
   // 1e-12 their rounding is all a rotation would resolve)
   const double jrel = s.phase == 0 ? kJacobiRel32 : (prm.mixed ? kJacobiRelMx : kJacobiRel64);
 
-  // 2. Gram matrices of the dot (summed over its chunks by dot_reduce_kernel)
+  // 2. Gram matrices of the dot (summed over its chunks by dot_reduce_kernel),
+  //    symmetrised and scaled to a unit diagonal of B
   const double *gsum = partial + size_t(d) * 2 * m * m;
-  for (int idx = tid; idx < m * m; idx += nt) {
-    sT[idx] = gsum[idx];
-    sZ[idx] = gsum[m * m + idx];
-  }
-  __syncthreads();
   const bool has_p = s.has_p != 0;
   if (tid < m) {
-    const double bii = sZ[tid * m + tid];
+    const double bii = gsum[m * m + tid * m + tid];
     const bool use = (has_p || tid < 2 * B) && bii > 0.0 && isfinite(bii);
     sD[tid] = use ? rsqrt(bii) : 0.0;
   }
   __syncthreads();
-  for (int idx = tid; idx < m * m; idx += nt) {
-    const int i = idx / m, j = idx % m;
-    const double dd = sD[i] * sD[j];
-    sA[idx] = 0.5 * (sT[i * m + j] + sT[j * m + i]) * dd;
-    sB[idx] = 0.5 * (sZ[i * m + j] + sZ[j * m + i]) * dd;
-  }
-  __syncthreads();
+  auto gram_at = [&](const double *G, int i, int j) {
+    return 0.5 * (G[i * m + j] + G[j * m + i]) * (sD[i] * sD[j]);
+  };
   // 3. Orthonormal basis of span[X W P] in the scaled B-inner product, as
-  //    Q (m x r) in sT.  FP32 phase: Cholesky B' = L L^T (outer-product form,
-  //    one barrier per column) and Q = L^-T, as long as every pivot stays above
-  //    kCholPivot32 (the scaled Gram has a unit diagonal, so a pivot is the
-  //    squared distance of a basis vector from the span of the previous ones);
-  //    likewise in the mixed form's finishing phase above kCholPivotMx.
-  //    Otherwise, and always in the plain FP64 form: SVQB (Jacobi on B', drop
-  //    directions with S < tau max S, Q = U_keep S_keep^-1/2).
-  bool chol = false;
-  if (s.phase == 0 || prm.mixed) {
+  //    Q in sT, and the projected matrix T = Q^T A' Q in registers.  Cholesky
+  //    (chol_congruence), as long as every pivot stays above the phase's floor
+  //    (the scaled Gram has a unit diagonal, so a pivot is the squared distance
+  //    of a basis vector from the span of the previous ones).  A direction of
+  //    P below it lies within sqrt(floor) of that span: it is dropped, its row
+  //    and column of T decoupled with a diagonal above the spectrum.  A small
+  //    pivot of X or W sends the basis to SVQB (Jacobi on B', directions with
+  //    S < tau max S dropped, Q = U_keep S_keep^-1/2).
+  constexpr int TM = (m + 15) / 16, S = 16 * TM;
+  Tile<TM> T;
+  int r = m;          // order of T
+  const int tx = tid & 15, ty = tid >> 4;
+  bool chol = true;
+  {
     const double pivot_floor = s.phase == 0 ? kCholPivot32 : kCholPivotMx;
     const int mu = has_p ? m : 2 * B;
-    bool usable = true;
-    for (int i = 0; i < mu; ++i) usable = usable && sD[i] > 0.0;
-    if (usable) {
-      for (int idx = tid; idx < m * m; idx += nt) sZ[idx] = sB[idx];
-      __syncthreads();
-      // A direction of P whose pivot falls below the floor lies within
-      // sqrt(floor) of the span of the columns before it: it is dropped (its
-      // column takes no part in the elimination); a small pivot of X or W
-      // sends the basis to SVQB.
-      bool ok = true;
-      int r = 0;   // kept columns, in order, in s_keep
-      for (int k = 0; k < mu; ++k) {
-        const double piv = sZ[k * m + k];   // final since the previous barrier
-        if (!(piv > pivot_floor)) {         // every thread reads the same value
-          if (k >= 2 * B) continue;
-          ok = false;
-          break;
+    for (int i = 0; i < mu; ++i) chol = chol && sD[i] > 0.0;
+    if (chol) {
+      Tile<TM> Bt, N;
+#pragma unroll
+      for (int a = 0; a < TM; ++a)
+#pragma unroll
+        for (int b = 0; b < TM; ++b) {
+          const int i = ty + 16 * a, j = tx + 16 * b;
+          const bool in = i < mu && j < mu;
+          T.v[a][b] = in ? gram_at(gsum, i, j) : 0.0;
+          Bt.v[a][b] = in ? gram_at(gsum + m * m, i, j) : 0.0;
+          N.v[a][b] = i == j ? 1.0 : 0.0;
         }
-        if (tid == 0) s_keep[r] = k;
-        ++r;
-        const double ip = 1.0 / piv;
-        const int R = mu - k - 1;
-        for (int idx = tid; idx < R * R; idx += nt) {
-          const int i = k + 1 + idx / R, j = k + 1 + idx % R;
-          if (j <= i) sZ[i * m + j] -= sZ[i * m + k] * sZ[j * m + k] * ip;
-        }
+      double *s_piv = sE;      // [m]
+      chol = chol_congruence<TM>(Bt, T, N, mu, 2 * B, pivot_floor, sW, s_piv);
+      if (chol) {
+        // the diagonal factor; Q[i][c] = N[c][i] / sqrt(piv_c)
+        if (tid < S) s_red[tid] = tid < mu && s_piv[tid] > 0.0 ? rsqrt(s_piv[tid]) : 0.0;
         __syncthreads();
-      }
-      if (ok) {
-        __syncthreads();   // s_keep complete
-        // L of the kept columns (r x r): L[c][c] = sqrt(piv), L[i][c] =
-        // Z[K_i][K_c] / sqrt(piv_c) into sT; 1/L[c][c] in sE
-        if (tid < r) sE[tid] = rsqrt(sZ[s_keep[tid] * m + s_keep[tid]]);
-        __syncthreads();
-        for (int idx = tid; idx < r * r; idx += nt) {
-          const int i = idx / r, c = idx % r;
-          if (c < i) sT[i * m + c] = sZ[s_keep[i] * m + s_keep[c]] * sE[c];
-        }
-        __syncthreads();
-        // L^-1 (lower) into sB, one column per thread
-        if (tid < r) {
-          const int j = tid;
-          for (int i = 0; i < j; ++i) sB[i * m + j] = 0.0;
-          sB[j * m + j] = sE[j];
-          for (int i = j + 1; i < r; ++i) {
-            double sum = 0.0;
-            for (int l = j; l < i; ++l) sum += sT[i * m + l] * sB[l * m + j];
-            sB[i * m + j] = -sum * sE[i];
+        double fro = 0.0;
+#pragma unroll
+        for (int a = 0; a < TM; ++a)
+#pragma unroll
+          for (int b = 0; b < TM; ++b) {
+            const int i = ty + 16 * a, j = tx + 16 * b;
+            const double si = s_red[i];
+            T.v[a][b] = si != 0.0 && s_red[j] != 0.0 ? T.v[a][b] * (si * s_red[j]) : 0.0;
+            fro = fma(T.v[a][b], T.v[a][b], fro);
+            if (i < m && j < m) sT[j * m + i] = si != 0.0 ? N.v[a][b] * si : 0.0;
           }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
+        if ((tid & 31) == 0) sW[tid >> 5] = fro;
+        __syncthreads();
+        fro = 0.0;
+        for (int w = 0; w < nt / 32; ++w) fro += sW[w];
+        const double above = 2.0 * sqrt(fro) + 1e-300;
+#pragma unroll
+        for (int a = 0; a < TM; ++a) {
+          const int i = ty + 16 * a;
+          if (tx == ty && i < m && s_red[i] == 0.0) T.v[a][a] = above;
         }
-        __syncthreads();
-        // Q = L^-T on the kept rows (m x r; dropped and unused rows zero)
-        for (int idx = tid; idx < m * m; idx += nt) sT[idx] = 0.0;
-        __syncthreads();
-        for (int idx = tid; idx < r * r; idx += nt) {
-          const int i = idx / r, c = idx % r;
-          if (c >= i) sT[s_keep[i] * m + c] = sB[c * m + i];
-        }
-        if (tid == 0) s_r = r;
-        __syncthreads();
-        chol = true;
-      } else {
         __syncthreads();
       }
     }
+  }
+  if (!chol) {
+    for (int idx = tid; idx < m * m; idx += nt) {
+      const int i = idx / m, j = idx % m;
+      sA[idx] = gram_at(gsum, i, j);
+      sB[idx] = gram_at(gsum + m * m, i, j);
+    }
+    __syncthreads();
   }
   if (!chol) {
     jacobi_cta(sB, sZ, m, m, jrel, s_red, s_c, s_s, s_p, s_q);
@@ -1529,7 +1668,7 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
       s_r = r;
     }
     __syncthreads();
-    const int r = s_r;
+    r = s_r;
     if (r < B || !(r > 0)) {
       if (tid == 0) {
         s.active = 0;
@@ -1550,35 +1689,37 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
     }
     __syncthreads();
   }
-  const int r = s_r;
-  // sZ = A' Q (m x r);  sB = Q^T sZ (r x r)
-  for (int idx = tid; idx < m * r; idx += nt) {
-    const int i = idx / r, c = idx % r;
-    double sum = 0.0;
-    for (int l = 0; l < m; ++l) sum += sA[i * m + l] * sT[l * m + c];
-    sZ[i * m + c] = sum;
-  }
-  __syncthreads();
-  for (int idx = tid; idx < r * r; idx += nt) {
-    const int i = idx / r, j = idx % r;
-    double sum = 0.0;
-    for (int l = 0; l < m; ++l) sum += sT[l * m + i] * sZ[l * m + j];
-    sB[i * m + j] = sum;
-  }
-  __syncthreads();
-  for (int idx = tid; idx < r * r; idx += nt) {
-    const int i = idx / r, j = idx % r;
-    if (i < j) {
-      const double v = 0.5 * (sB[i * m + j] + sB[j * m + i]);
-      sB[i * m + j] = v;
-      sB[j * m + i] = v;
+  if (!chol) {
+    // sZ = A' Q (m x r);  sB = Q^T sZ (r x r)
+    for (int idx = tid; idx < m * r; idx += nt) {
+      const int i = idx / r, c = idx % r;
+      double sum = 0.0;
+      for (int l = 0; l < m; ++l) sum += sA[i * m + l] * sT[l * m + c];
+      sZ[i * m + c] = sum;
     }
+    __syncthreads();
+    for (int idx = tid; idx < r * r; idx += nt) {
+      const int i = idx / r, j = idx % r;
+      double sum = 0.0;
+      for (int l = 0; l < m; ++l) sum += sT[l * m + i] * sZ[l * m + j];
+      sB[i * m + j] = sum;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < TM; ++a)
+#pragma unroll
+      for (int b = 0; b < TM; ++b) {
+        const int i = ty + 16 * a, j = tx + 16 * b;
+        T.v[a][b] = i < r && j < r ? 0.5 * (sB[i * m + j] + sB[j * m + i]) : 0.0;
+      }
+    __syncthreads();
   }
-  __syncthreads();
-  // 4. the B lowest eigenpairs of the standard problem of size r: values
-  //    ascending into sE, vectors into sA's first B columns (sZ is free
-  //    scratch now)
-  tridiag_lowest_cta(sB, sA, r, m, B, sE, sZ, sW);
+  // 4. the B lowest eigenpairs of the standard problem of order r: values
+  //    ascending into sE, vectors into sV (sA and sB are free scratch now, the
+  //    reflectors go to sZ)
+  constexpr int ldv = B + 1;
+  double *sV = sA + 12 * B * B;
+  tridiag_lowest_cta<TM>(T, sV, ldv, r, B, sE, sA, sZ, sW);
   if (tid < B) s_sel[tid] = tid;
   __syncthreads();
   // 5. Y = D Q Z[:, sel]  (m x B)
@@ -1587,7 +1728,7 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
     const int i = idx / B, c = idx % B;
     const int zc = s_sel[c];
     double sum = 0.0;
-    for (int l = 0; l < r; ++l) sum += sT[i * m + l] * sA[l * m + zc];
+    for (int l = 0; l < r; ++l) sum += sT[i * m + l] * sV[l * ldv + zc];
     Y[idx] = sD[i] * sum;
   }
   if (tid < B) th[tid] = sE[s_sel[tid]];
@@ -2353,7 +2494,10 @@ struct Layout {
 
 size_t rr_smem_bytes(int B) {
   const int m = 3 * B;
-  return size_t(4 * m * m + 2 * m + B + 4 * m + 256 + 3 * B) * sizeof(double);
+  const int S = (m + 15) / 16 * 16;
+  // A', B', Q, reflectors (order r <= m, rows of S), scaling, eigenvalues,
+  // residuals, scratch (also the 16 B chunk sums of the residual norms)
+  return size_t(3 * m * m + m * S + 2 * S + B + 10 * S + 16) * sizeof(double);
 }
 
 int carve(qd::Arena &ar, int n_dots, int64_t n_rows, int64_t nnz, int B, int nchunks,
