@@ -51,6 +51,12 @@ constexpr int kJRows = kMaxU / kJC;  // rows of Z per CTA (18)
 constexpr int kJThreads = 512;
 constexpr double kSchurTol = 1e-14;   // |c_qp| <= kSchurTol ||C||_F counts as zero
 constexpr int kSchurSweeps = 60;
+// SVQB drops directions whose eigenvalue of the scaled Gram matrix is below this
+// share of the largest: what is kept is scaled up by its inverse square root, and
+// with it the rounding of P's products, which come from combination.  At 1e-14
+// (factors of 1e7) one late SVQB step could set off a growth of the residuals by
+// a factor of three per iteration; 1e-10 takes the same iterations without it.
+constexpr double kDrop64 = 1e-10, kDrop32 = 1e-6;
 
 template <typename T> struct CT;
 template <> struct CT<float> { using type = float2; };
@@ -1426,7 +1432,7 @@ extern "C" int qd_cap_lobpcg_solve(int32_t n, const int32_t *d_rowptr, const int
     cap_init_kernel<float2><<<grid_for(int64_t(n) * b, 256), 256, 0, s>>>(
         n, b, ld, seed, static_cast<float2 *>(w.b32.S[0]));
     QD_CHECK_LAUNCH();
-    st = lobpcg_run<float>(P, w, w.b32, cur32, tol32, max_iter, 8, 1e-6, res, it32, &sweeps, &unconv);
+    st = lobpcg_run<float>(P, w, w.b32, cur32, tol32, max_iter, 8, kDrop32, res, it32, &sweeps, &unconv);
     if (st != QD_OK) return st;
     double r32 = 0.0;
     for (int j = 0; j < nev; ++j) r32 = std::max(r32, res[j]);
@@ -1445,7 +1451,7 @@ extern "C" int qd_cap_lobpcg_solve(int32_t n, const int32_t *d_rowptr, const int
     QD_CHECK_LAUNCH();
   }
   int it64 = 0;
-  st = lobpcg_run<double>(P, w, w.b64, cur64, tol, max_iter, 0, 1e-14, res, it64, &sweeps, &unconv);
+  st = lobpcg_run<double>(P, w, w.b64, cur64, tol, max_iter, 0, kDrop64, res, it64, &sweeps, &unconv);
   if (st != QD_OK) return st;
   h_info->iters_fp64 = it64;
   h_info->schur_sweeps_max = sweeps;
