@@ -48,7 +48,7 @@ constexpr int kMaxB = 48;            // largest block (3b <= 144)
 constexpr int kMaxU = 3 * kMaxB;     // leading dimension of every small matrix
 constexpr int kJC = 8;               // CTAs per cluster of the Schur kernel
 constexpr int kJRows = kMaxU / kJC;  // rows of Z per CTA (18)
-constexpr int kJThreads = 512;
+constexpr int kJThreads = 672;       // one 2 x 2 block of the largest problem each (9 x 72)
 constexpr double kSchurTol = 1e-14;   // |c_qp| <= kSchurTol ||C||_F counts as zero
 constexpr int kSchurSweeps = 60;
 // SVQB drops directions whose eigenvalue of the scaled Gram matrix is below this
@@ -57,6 +57,8 @@ constexpr int kSchurSweeps = 60;
 // (factors of 1e7) one late SVQB step could set off a growth of the residuals by
 // a factor of three per iteration; 1e-10 takes the same iterations without it.
 constexpr double kDrop64 = 1e-10, kDrop32 = 1e-6;
+// rotations (u1, u2) of a solve of the largest order and most sweeps: 20 MB
+constexpr size_t kSchurLog = size_t(kSchurSweeps) * (kMaxU - 1) * kMaxU;
 
 template <typename T> struct CT;
 template <> struct CT<float> { using type = float2; };
@@ -554,36 +556,64 @@ cap_small_gemm_kernel(int m, int nn, int k, const int *m_dev, const int *n_dev, 
 // Hermitian input the result is its eigendecomposition (T diagonal).
 //
 // Cluster of kJC CTAs.  The pairs are split into kJC contiguous ranges, and
-// CTA r keeps the rows of C of the indices paired in its range, so that a
-// pair's 2 x 2 block and both of its rows are local.  Round-robin order as
-// a ring: index N-1 stays in pair 0, the other indices move one place per
-// round (the first member of pair k+1 to pair k, the second member of pair
-// k-1 to pair k; pair 0's moving member to pair 1, the last pair's second
-// member becomes its first), so only the two rows at each range boundary
-// change CTA per round.  Z's rows are split statically (only its columns
-// rotate).  Per round:
-//   (1) warp 0 forms the rotations of the CTA's pairs and writes them to
-//       every CTA; the other warps rotate Z's columns by the previous round's
-//       rotations;
-//   (2) cluster barrier; each CTA applies U_a^H B U_b to every 2 x 2 block B
-//       of its rows (rows of pair a, columns of pair b);
-//   (3) the boundary rows go to the neighbours' landing rows; cluster
-//       barrier; each CTA moves the landed rows into the freed slots.
+// CTA r keeps the rows of C of the indices paired in its range of the
+// round-robin order, a ring: index N-1 stays in pair 0, the other indices move
+// one place per round (the first member of pair k+1 to pair k, the second
+// member of pair k-1 to pair k; pair 0's moving member to pair 1, the last
+// pair's second member becomes its first), so only the two rows at each range
+// boundary change CTA per round, into a slot that its receiver keeps free and
+// has told its neighbour.  The index at place s of the ring in round g is
+// (g - s) mod (N - 1), so every CTA knows all pairs.  Z's rows are split
+// statically (only its columns rotate).  Per round:
+//   (1) every CTA forms the rotations of all pairs from the four elements of
+//       each pair's 2 x 2 block;
+//   (2) it applies U_a^H B U_b to every 2 x 2 block B of its rows (rows of pair
+//       a, columns of pair b);
+//   (3) each row sends its two elements of the next round's 2 x 2 block to every
+//       CTA, and the boundary rows go to the neighbours;
+//   (4) cluster barrier; the rotations go to a log, from which cap_schur_z_kernel
+//       forms Z on other SMs afterwards (without a log Z is rotated here).
 // Every thread of every CTA passes the same barriers (the loop bounds and
 // the stop test are cluster-uniform).
+// The latency of the chain bounds it: of a round's 4.4k cycles the rotations
+// take 1.0k, the blocks 1.3k (half of it FP64 issue), the messages 0.65k and
+// the barrier with their arrival 1.2k.  With the rotations formed by their
+// pair's CTA only and sent round, which takes a second cluster barrier, and Z
+// rotated in the kernel a round took 3.5 us at n = 144; now 2.1 us, and 0.2 us
+// of cap_schur_z_kernel.  Updating only the blocks that the messages need
+// first, and the others while these travel, gains nothing (375 and 386 ms a
+// solve against 372).
 // ---------------------------------------------------------------------------
 struct Rot {
   double2 u1, u2;   // U = [[u1, -conj(u2)], [u2, conj(u1)]]
-  int on, p, q, pad;
+  int on, p, q, mp; // p < q; mp: which member of the pair p is
 };
 
 constexpr int kJPairs = kMaxU / 2 / kJC;     // pairs per CTA (9)
-constexpr int kJSlots = 2 * kJPairs + 2;     // rows of C per CTA: pairs' rows + 2 landing rows
-constexpr int kLandL = 2 * kJPairs, kLandR = 2 * kJPairs + 1;
+constexpr int kJSlots = 2 * kJPairs + 2;     // rows of C per CTA: pairs' rows + 2 free ones
 constexpr size_t kJSmem = size_t(kJSlots) * kMaxU * sizeof(double2) +     // C rows
                           size_t(kJRows) * kMaxU * sizeof(double2) +      // Z rows
-                          2 * (kMaxU / 2) * sizeof(Rot) +
-                          (2 * kJPairs + kJSlots + 4) * sizeof(int) + 2 * sizeof(double) + 64;
+                          2 * (kMaxU / 2) * sizeof(Rot) +                 // by round parity
+                          2 * kMaxU * 2 * sizeof(double2);   // [parity][pair][member] elements
+
+// Place (k, m) of the ring: the index there in round g (gm = g mod M), and the
+// place it moves to.
+__device__ __forceinline__ int ring_index(int k, int m, int gm, int M) {
+  if (k == 0) return m == 0 ? M : gm;
+  const int i = m == 1 ? gm - k : gm + k;
+  return i < 0 ? i + M : (i >= M ? i - M : i);
+}
+__device__ __forceinline__ void ring_next(int k, int m, int K, int &nk, int &nm) {
+  if (k == 0 && m == 0) {
+    nk = 0; nm = 0;
+  } else if (m == 1) {
+    nk = k < K ? k + 1 : K;
+    nm = k < K || K == 0 ? 1 : 0;
+  } else {
+    nk = k > 1 ? k - 1 : 0;
+    nm = k > 1 ? 0 : 1;
+  }
+}
 
 __device__ __forceinline__ Rot make_rot(double2 a, double2 bb, double2 c, double2 d, double thresh2,
                                         int p, int q) {
@@ -593,18 +623,19 @@ __device__ __forceinline__ Rot make_rot(double2 a, double2 bb, double2 c, double
   R.on = 0;
   R.p = p;
   R.q = q;
-  R.pad = 0;
+  R.mp = 0;
   if (cabs2(c) > thresh2) {
     // eigenvalue lambda of the 2 x 2 block nearer a: with h = (a - d)/2,
     // disc = sqrt(h^2 + b c), lambda - a = b c / g, g the larger of h +- disc
     // (entries are O(||C||), far from the FP64 range limits: plain formulas)
     const double2 h = cscale(csub(a, d), 0.5);
     const double2 z = cadd(cmul(h, h), cmul(bb, c));
-    const double r = sqrt(cabs2(z));
+    // square roots and quotients by reciprocals: their latency is the chain's
+    const double z2 = cabs2(z);
     double2 disc = make_double2(0.0, 0.0);
-    if (r > 0.0) {
-      const double t = sqrt(0.5 * (r + fabs(z.x)));
-      const double v = 0.5 * z.y / t;
+    if (z2 > 0.0) {
+      const double w = 0.5 * (z2 * rsqrt(z2) + fabs(z.x)), it = rsqrt(w);
+      const double t = w * it, v = 0.5 * z.y * it;
       disc = z.x >= 0.0 ? make_double2(t, v) : make_double2(fabs(v), copysign(t, z.y));
     }
     const double2 g1 = cadd(h, disc), g2 = csub(h, disc);
@@ -625,7 +656,7 @@ __global__ void __cluster_dims__(kJC, 1, 1) __launch_bounds__(kJThreads, 1)
 cap_schur_kernel(int n_fix, const int *__restrict__ n_dev, const int *__restrict__ skip_if_set,
                  const double2 *__restrict__ Cin, int ldi, double2 *__restrict__ Tout,
                  double2 *__restrict__ Zout, int ldo, int max_sweeps, double rel_tol,
-                 int *__restrict__ sweeps_out) {
+                 int *__restrict__ sweeps_out, double2 *__restrict__ log) {
   cg::cluster_group cluster = cg::this_cluster();
   // uniform early exit (every CTA reads the same flag before any barrier)
   if (skip_if_set && *skip_if_set) return;
@@ -640,30 +671,24 @@ cap_schur_kernel(int n_fix, const int *__restrict__ n_dev, const int *__restrict
   extern __shared__ __align__(16) unsigned char jsm[];
   double2 *Cs = reinterpret_cast<double2 *>(jsm);
   double2 *Zl = Cs + size_t(kJSlots) * kMaxU;
-  Rot *rot = reinterpret_cast<Rot *>(Zl + size_t(kJRows) * kMaxU);   // [2][kMaxU / 2]
-  int *pos = reinterpret_cast<int *>(rot + 2 * (kMaxU / 2));         // [2 kJPairs] slot of (pair, member)
-  int *idx = pos + 2 * kJPairs;                                       // [kJSlots] index held by a slot
-  int *s_cnt = idx + kJSlots;                                         // [2] rotations this sweep
-  double *s_norm = reinterpret_cast<double *>(s_cnt + 4);
-  __shared__ double s_w[kJThreads / 32];
-  __shared__ int s_new[2 * kJPairs], s_fill[2][2];
+  Rot *rots = reinterpret_cast<Rot *>(Zl + size_t(kJRows) * kMaxU);  // [2][kMaxU / 2], by round parity
+  double2 *elem = reinterpret_cast<double2 *>(rots + kMaxU);         // [2][pair][member](self, partner)
+  __shared__ double s_w[kJThreads / 32], s_norm[1];
+  __shared__ int pos[2][2 * kJPairs];     // slot of (pair, member), by round parity
+  __shared__ int spare[2][2];             // free slot for the row from the left / right
+  __shared__ int nbr[2][2];               // the left neighbour's for its right, the right one's
 
   const int k0 = rank * P, k1 = min(npairs, k0 + P), np = max(0, k1 - k0);
   const int z0 = rank * RZ, nz = max(0, min(RZ, N - z0));
-  // round-0 positions: pair 0 = (M, 0), pair k = (k, M - k)
-  if (tid < 2 * np) {
-    const int k = k0 + tid / 2, m = tid & 1;
-    pos[tid] = tid;
-    idx[tid] = k == 0 ? (m == 0 ? M : 0) : (m == 0 ? k : M - k);
+  const bool out_l = np > 0 && k0 >= 1, out_r = np > 0 && k1 - 1 < K;
+  if (tid < 2 * np) pos[0][tid] = tid;
+  if (tid < 2) {
+    spare[0][tid] = 2 * kJPairs + tid;
+    nbr[0][tid] = 2 * kJPairs + 1 - tid;
   }
-  if (tid == 0) {
-    s_cnt[0] = s_cnt[1] = 0;
-    idx[kLandL] = idx[kLandR] = -1;
-  }
-  __syncthreads();
   double nrm = 0.0;
   for (int e = tid; e < 2 * np * N; e += kJThreads) {
-    const int sl = e / N, j = e % N, i = idx[sl];
+    const int sl = e / N, j = e % N, i = ring_index(k0 + sl / 2, sl & 1, 0, M);
     const double2 v = (i < n && j < n) ? Cin[size_t(i) * ldi + j] : make_double2(0.0, 0.0);
     Cs[sl * kMaxU + j] = v;
     nrm += cabs2(v);
@@ -681,66 +706,89 @@ cap_schur_kernel(int n_fix, const int *__restrict__ n_dev, const int *__restrict
     for (int w = 0; w < kJThreads / 32; ++w) sacc += s_w[w];
     s_norm[0] = sacc;
   }
+  // the elements (i, i), (i, j) of the row of place (k0 + t, m), whose index i is
+  // paired with j next, to CTA dst's table
+  auto send_elem = [&](int t, int m, int slot, int i, int nk, int nm, int j, int buf, int dst) {
+    double2 *to = dst == rank ? elem : cluster.map_shared_rank(elem, dst);
+    to += (buf * kMaxU + 2 * nk + nm) * 2;
+    to[0] = Cs[slot * kMaxU + i];
+    to[1] = Cs[slot * kMaxU + j];
+  };
+  for (int e = tid; e < 2 * np * kJC; e += kJThreads) {
+    const int sl = e / kJC, k = k0 + sl / 2, m = sl & 1;
+    send_elem(sl / 2, m, sl, ring_index(k, m, 0, M), k, m, ring_index(k, 1 - m, 0, M), 0, e % kJC);
+  }
   cluster.sync();
   double fro2 = 0.0;
   for (int r = 0; r < kJC; ++r) fro2 += *cluster.map_shared_rank(s_norm, r);
   const double thresh2 = rel_tol * rel_tol * fro2;
-
-  // Z <- Z U for the rotations of one round (rotation table `par`)
-  // items (row, pair) spread evenly over threads t0..t0+nt-1; the quotient
-  // by npairs in single precision is exact for these small integers
+  // item numbers to (row, pair): the quotient by npairs in single precision is
+  // exact for these small integers
   const float inv_np = 1.0f / float(npairs);
-  auto rotate_z = [&](int par, int t0, int nt) {
-    for (int e = tid - t0; e < nz * npairs; e += nt) {
-      const int li = int((float(e) + 0.5f) * inv_np), k = e - li * npairs;
-      const Rot &R = rot[par * (kMaxU / 2) + k];
-      if (!R.on) continue;
-      double2 *z = Zl + li * kMaxU;
-      const double2 x = z[R.p], y = z[R.q];
-      z[R.p] = cadd(cmul(x, R.u1), cmul(y, R.u2));
-      z[R.q] = csub(cmul(y, cconj(R.u1)), cmul(x, cconj(R.u2)));
-    }
-  };
 
+  // this thread's part in step (3), the same in every round: elements of a row
+  // for one CTA (w < ne), one entry of a boundary row, or one place's slot
+  const int ne = 2 * np * kJC;
+  int role = -1, ra = 0, rb = 0, rk = 0, rm = 0, nk = 0, nm = 0;
+  double2 *peer = nullptr;
+  int *peer_nbr = nullptr;
+  if (tid < ne) {
+    role = 0;
+    ra = tid / kJC;                        // local row: (pair, member)
+    rk = k0 + (ra >> 1);
+    rm = ra & 1;
+    ring_next(rk, rm, K, nk, nm);
+    peer = cluster.map_shared_rank(elem, tid % kJC) + (2 * nk + nm) * 2;
+  } else if (tid < ne + 2 * N) {
+    const int side = (tid - ne) / N;
+    if (side == 0 ? out_l : out_r) {
+      role = 1;
+      ra = side;
+      rb = (tid - ne) - side * N;          // column
+      rk = side == 0 ? 0 : 2 * (np - 1) + 1;
+      peer = cluster.map_shared_rank(Cs, side == 0 ? rank - 1 : rank + 1) + rb;
+      peer_nbr = cluster.map_shared_rank(&nbr[0][0], side == 0 ? rank - 1 : rank + 1) + 1 - side;
+    }
+  } else if (tid < ne + 2 * N + 2 * np) {
+    role = 2;
+    ra = tid - ne - 2 * N;
+    const int k = k0 + (ra >> 1), m = ra & 1;
+    // where the row of place (k, m) comes from
+    const int sk = m == 0 ? (k == 0 ? 0 : (k < K ? k + 1 : K)) : (k == 0 ? (K >= 1 ? 1 : 0) : k - 1);
+    const int sm = m == 0 ? (k == 0 || k < K ? 0 : 1) : (k == 0 && K >= 1 ? 0 : 1);
+    rb = sk >= k0 && sk < k1 ? 2 * (sk - k0) + sm : (sk < k0 ? -1 : -2);
+  }
+  static_assert(2 * kJPairs * kJC + 2 * kMaxU + 2 * kJPairs <= kJThreads, "one part per thread");
   int sweeps = 0, converged = N < 2;
-  int g = 0;   // rounds run
+  int gm = 0;                              // rounds run, mod M
+  double2 *log_at = log;
+  int par = 0;                             // rounds run, mod 2
   for (int sw = 0; sw < max_sweeps && N >= 2; ++sw) {
-    const int cpar = sw & 1;
-    for (int rr = 0; rr < N - 1; ++rr, ++g) {
-      const int par = g & 1;
-      // (1) rotations of my pairs (warp 0), Z by the previous round (others)
-      if (warp == 0) {
-        if (lane < np) {
-          const int k = k0 + lane;
-          int sp = pos[2 * lane], sq = pos[2 * lane + 1];
-          int p = idx[sp], q = idx[sq];
-          if (p > q) {
-            const int t = p; p = q; q = t;
-            const int u = sp; sp = sq; sq = u;
-          }
-          const Rot R = make_rot(Cs[sp * kMaxU + p], Cs[sp * kMaxU + q], Cs[sq * kMaxU + p],
-                                 Cs[sq * kMaxU + q], thresh2, p, q);
-          if (R.on) atomicAdd(&s_cnt[cpar], 1);
-          for (int dst = 0; dst < kJC; ++dst) {
-            Rot *rp = dst == rank ? rot : cluster.map_shared_rank(rot, dst);
-            rp[par * (kMaxU / 2) + k] = R;
-          }
-        }
-      } else if (g > 0) {
-        if (tid >= 64) rotate_z(par ^ 1, 64, kJThreads - 64);
+    int count = 0;                         // rotations this sweep
+    for (int rr = 0; rr < N - 1; ++rr) {
+      const int gn = gm + 1 == M ? 0 : gm + 1;
+      // a warp may be in the next round while others still rotate Z by this one
+      Rot *rot = rots + par * (kMaxU / 2);
+      // (1)
+      bool on = false;
+      if (tid < npairs) {
+        const int i0 = ring_index(tid, 0, gm, M), i1 = ring_index(tid, 1, gm, M);
+        const int mp = i0 < i1 ? 0 : 1;
+        const double2 *e = elem + (par * kMaxU + 2 * tid) * 2;
+        Rot R = make_rot(e[2 * mp], e[2 * mp + 1], e[2 * (1 - mp) + 1], e[2 * (1 - mp)], thresh2,
+                         min(i0, i1), max(i0, i1));
+        R.mp = mp;
+        rot[tid] = R;
+        on = R.on != 0;
       }
-      cluster.sync();
+      count += __syncthreads_count(on);
       // (2) 2 x 2 blocks of my rows: U_a^H B U_b
       for (int e = tid; e < np * npairs; e += kJThreads) {
         const int t = int((float(e) + 0.5f) * inv_np), kb = e - t * npairs;
-        const Rot &Ra = rot[par * (kMaxU / 2) + k0 + t];
-        const Rot &Rb = rot[par * (kMaxU / 2) + kb];
+        const Rot &Ra = rot[k0 + t];
+        const Rot &Rb = rot[kb];
         if (!Ra.on && !Rb.on) continue;
-        int sp = pos[2 * t], sq = pos[2 * t + 1];
-        if (idx[sp] != Ra.p) {
-          const int u = sp; sp = sq; sq = u;
-        }
-        double2 *rp = Cs + sp * kMaxU, *rq = Cs + sq * kMaxU;
+        double2 *rp = Cs + pos[par][2 * t + Ra.mp] * kMaxU, *rq = Cs + pos[par][2 * t + 1 - Ra.mp] * kMaxU;
         double2 x0 = rp[Rb.p], x1 = rp[Rb.q], y0 = rq[Rb.p], y1 = rq[Rb.q];
         if (Ra.on) {   // rows: [p; q] <- U_a^H [p; q]
           const double2 nx0 = cadd(cmulc(Ra.u1, x0), cmulc(Ra.u2, y0));
@@ -764,87 +812,60 @@ cap_schur_kernel(int n_fix, const int *__restrict__ n_dev, const int *__restrict
         rq[Rb.q] = y1;
       }
       __syncthreads();
-      // (3) ring shift: member 0 of my first pair goes left, member 1 of my
-      // last pair goes right (each to the neighbour's landing row)
-      const bool out_l = np > 0 && k0 >= 1, out_r = np > 0 && k1 - 1 < K;
-      if (out_l || out_r) {
-        for (int e = tid; e < 2 * N; e += kJThreads) {
-          const int side = e / N, j = e % N;
-          if (side == 0 ? !out_l : !out_r) continue;
-          const int src = side == 0 ? pos[0] : pos[2 * (np - 1) + 1];
-          const int dst_rank = side == 0 ? rank - 1 : rank + 1;
-          double2 *peer = cluster.map_shared_rank(Cs, dst_rank);
-          peer[(side == 0 ? kLandR : kLandL) * kMaxU + j] = Cs[src * kMaxU + j];
-          if (j == 0) cluster.map_shared_rank(idx, dst_rank)[side == 0 ? kLandR : kLandL] = idx[src];
+      // (3) elements to every CTA, boundary rows to the neighbours, and the
+      // places of the next round
+      if (role == 0) {
+        const int i = ring_index(rk, rm, gm, M), j = ring_index(nk, 1 - nm, gn, M);
+        const double2 *row = Cs + pos[par][ra] * kMaxU;
+        double2 *to = peer + (par ^ 1) * kMaxU * 2;
+        to[0] = row[i];
+        to[1] = row[j];
+      } else if (role == 1) {
+        const int src = pos[par][rk];
+        peer[nbr[par][ra] * kMaxU] = Cs[src * kMaxU + rb];
+        if (rb == 0) {   // the slot it leaves is the next free one on this side
+          spare[par ^ 1][ra] = src;
+          peer_nbr[(par ^ 1) * 2] = src;
         }
+      } else if (role == 2) {
+        pos[par ^ 1][ra] = rb >= 0 ? pos[par][rb] : spare[par][rb == -1 ? 0 : 1];
       }
-      if (K >= 1) {
-        // new slot of every position (k, m), k in my range (one thread each):
-        // the source position's slot if local, else a landing row, moved into
-        // the slot freed by the row that left on the same side
-        if (tid < 2) s_fill[tid][0] = -1;
-        __syncthreads();
-        if (tid < 2 * np) {
-          const int t = tid >> 1, m = tid & 1, k = k0 + t;
-          int sk, sm;   // source position
-          if (m == 0) {
-            if (k == 0) { sk = 0; sm = 0; }
-            else if (k < K) { sk = k + 1; sm = 0; }
-            else { sk = K; sm = 1; }
-          } else {
-            if (k == 0) { sk = 1; sm = 0; }
-            else if (k == 1) { sk = 0; sm = 1; }
-            else { sk = k - 1; sm = 1; }
-          }
-          int slot;
-          if (sk >= k0 && sk < k1) {
-            slot = pos[2 * (sk - k0) + sm];
-          } else if (sk < k0) {   // arrives from the left
-            slot = pos[0];
-            s_fill[0][0] = kLandL;
-            s_fill[0][1] = slot;
-          } else {                 // arrives from the right
-            slot = pos[2 * (np - 1) + 1];
-            s_fill[1][0] = kLandR;
-            s_fill[1][1] = slot;
-          }
-          s_new[tid] = slot;
+      // (4) between arrival and wait: the rotations to the log, from which
+      // cap_schur_z_kernel forms Z, or without one Z <- Z U (items (row, pair))
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+      if (log) {
+        if (tid < npairs && rank == (gm & (kJC - 1))) {
+          log_at[2 * tid] = rot[tid].u1;
+          log_at[2 * tid + 1] = rot[tid].u2;
         }
+        log_at += 2 * npairs;
       }
-      cluster.sync();
-      // landed rows into the freed slots, then the new positions
-      if (K >= 1) {
-        for (int e = tid; e < 2 * N; e += kJThreads) {
-          const int side = e / N, j = e % N;
-          const int from = s_fill[side][0];
-          if (from < 0) continue;
-          const int to = s_fill[side][1];
-          Cs[to * kMaxU + j] = Cs[from * kMaxU + j];
-          if (j == 0) idx[to] = idx[from];
-        }
-        if (tid < 2 * np) pos[tid] = s_new[tid];
+      for (int e = tid; !log && e < nz * npairs; e += kJThreads) {
+        const int li = int((float(e) + 0.5f) * inv_np), k = e - li * npairs;
+        const Rot &R = rot[k];
+        if (!R.on) continue;
+        double2 *z = Zl + li * kMaxU;
+        const double2 x = z[R.p], y = z[R.q];
+        z[R.p] = cadd(cmul(x, R.u1), cmul(y, R.u2));
+        z[R.q] = csub(cmul(y, cconj(R.u1)), cmul(x, cconj(R.u2)));
       }
-      __syncthreads();
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+      gm = gn;
+      par ^= 1;
     }
     ++sweeps;
-    int total = 0;
-    for (int r = 0; r < kJC; ++r) total += cluster.map_shared_rank(s_cnt, r)[cpar];
-    cluster.sync();   // every CTA has read the counters
-    if (tid == 0) s_cnt[cpar] = 0;
-    __syncthreads();
-    if (total == 0) {
+    if (count == 0) {
       converged = 1;
       break;
     }
   }
-  if (g > 0) rotate_z((g - 1) & 1, 0, kJThreads);   // the last round's rotations
-  __syncthreads();
   for (int e = tid; e < 2 * np * N; e += kJThreads) {
-    const int sl = e / N, j = e % N;
-    const int s_ = pos[sl], i = idx[s_];
-    if (i < n && j < n) Tout[size_t(i) * ldo + j] = Cs[s_ * kMaxU + j];
+    const int sl = e / N, j = e % N, i = ring_index(k0 + sl / 2, sl & 1, gm, M);
+    if (i < n && j < n) Tout[size_t(i) * ldo + j] = Cs[pos[par][sl] * kMaxU + j];
   }
-  for (int e = tid; e < nz * N; e += kJThreads) {
+  for (int e = tid; !log && e < nz * N; e += kJThreads) {
     const int li = e / N, j = e % N, i = z0 + li;
     if (i < n && j < n) Zout[size_t(i) * ldo + j] = Zl[li * kMaxU + j];
   }
@@ -853,6 +874,49 @@ cap_schur_kernel(int n_fix, const int *__restrict__ n_dev, const int *__restrict
     sweeps_out[1] = converged;
   }
   cluster.sync();   // no CTA leaves while a peer may still write to it
+}
+
+// Z from the log of a Schur solve's rotations: row i is e_i^T U_1 U_2 ..., and the
+// rows are independent, so a block takes one.  A thread per pair; its next
+// kZAhead rotations are on their way to shared memory.
+constexpr int kZThreads = 96;      // >= kMaxU / 2
+constexpr int kZAhead = 8;
+__global__ void __launch_bounds__(kZThreads)
+cap_schur_z_kernel(int n_fix, const int *__restrict__ n_dev, const int *__restrict__ skip_if_set,
+                   const int *__restrict__ sweeps, const double2 *__restrict__ log,
+                   double2 *__restrict__ Zout, int ldo) {
+  __shared__ double2 z[kMaxU], s_rot[kZAhead][kMaxU];
+  if (skip_if_set && *skip_if_set) return;
+  const int n = n_dev ? *n_dev : n_fix, row = blockIdx.x, tid = threadIdx.x;
+  if (row >= n) return;
+  const int N = n + (n & 1), M = N - 1, npairs = N / 2, rounds = *sweeps * M;
+  for (int j = tid; j < N; j += kZThreads) z[j] = make_double2(j == row ? 1.0 : 0.0, 0.0);
+  auto fetch = [&](int g) {
+    if (tid < npairs && g < rounds) {
+      const double2 *src = log + size_t(g) * 2 * npairs + 2 * tid;
+      cp_async16(&s_rot[g % kZAhead][2 * tid], src, 16);
+      cp_async16(&s_rot[g % kZAhead][2 * tid + 1], src + 1, 16);
+    }
+    cp_async_commit();
+  };
+  for (int g = 0; g < kZAhead - 1; ++g) fetch(g);
+  __syncthreads();
+  for (int g = 0, gm = 0; g < rounds; ++g, gm = gm + 1 == M ? 0 : gm + 1) {
+    fetch(g + kZAhead - 1);
+    cp_async_wait<kZAhead - 1>();              // a thread reads its own copies
+    if (tid < npairs) {
+      const double2 u1 = s_rot[g % kZAhead][2 * tid], u2 = s_rot[g % kZAhead][2 * tid + 1];
+      if (u2.x != 0.0 || u2.y != 0.0 || u1.x != 1.0 || u1.y != 0.0) {
+        const int i0 = ring_index(tid, 0, gm, M), i1 = ring_index(tid, 1, gm, M);
+        const int p = min(i0, i1), q = max(i0, i1);
+        const double2 x = z[p], y = z[q];
+        z[p] = cadd(cmul(x, u1), cmul(y, u2));
+        z[q] = csub(cmul(y, cconj(u1)), cmul(x, cconj(u2)));
+      }
+    }
+    __syncthreads();
+  }
+  for (int j = tid; j < n; j += kZThreads) Zout[size_t(row) * ldo + j] = z[j];
 }
 
 // ---------------------------------------------------------------------------
@@ -1138,6 +1202,7 @@ struct Work {
   double *dscale, *rpart, *res;
   double2 *theta, *bpart, *bsum, *E, *scale;
   int *nkeep, *ok, *status, *sel, *act, *pick, *sweeps;
+  double2 *log;              // rotations of one Schur solve
 };
 
 size_t carve(qd::Arena &ar, int32_t n, int b, bool mixed, size_t dst_bytes, Work &w) {
@@ -1182,7 +1247,8 @@ size_t carve(qd::Arena &ar, int32_t n, int b, bool mixed, size_t dst_bytes, Work
   w.sel = ar.take<int>(kMaxB);
   w.act = ar.take<int>(kMaxB);
   w.pick = ar.take<int>(kMaxB);
-  w.sweeps = ar.take<int>(2);   // largest sweep count, all converged
+  w.sweeps = ar.take<int>(4);   // sweeps and convergence of the last solve, and of the SVQB one
+  w.log = ar.take<double2>(kSchurLog);
   return ar.used;
 }
 
@@ -1242,7 +1308,9 @@ int lobpcg_run(const Problem &P, Work &w, Blocks &bl, int &cur, double tol, int 
     cap_svqb_prep_kernel<<<grid_for(u * u, 256), 256, 0, s>>>(u, w.ok, w.GM, w.dscale, w.J);
     QD_CHECK_LAUNCH();
     cap_schur_kernel<<<kJC, kJThreads, kJSmem, s>>>(u, nullptr, w.ok, w.J, kMaxU, w.T, w.Z, kMaxU,
-                                                    kSchurSweeps, kSchurTol, nullptr);
+                                                    kSchurSweeps, kSchurTol, w.sweeps + 2, w.log);
+    QD_CHECK_LAUNCH();
+    cap_schur_z_kernel<<<u, kZThreads, 0, s>>>(u, nullptr, w.ok, w.sweeps + 2, w.log, w.Z, kMaxU);
     QD_CHECK_LAUNCH();
     cap_svqb_finish_kernel<<<1, 256, 0, s>>>(u, drop, w.ok, w.T, w.Z, w.dscale, w.Bm, w.nkeep);
     QD_CHECK_LAUNCH();
@@ -1255,7 +1323,9 @@ int lobpcg_run(const Problem &P, Work &w, Blocks &bl, int &cur, double tol, int 
                                              kMaxU, w.C, kMaxU);
     QD_CHECK_LAUNCH();
     cap_schur_kernel<<<kJC, kJThreads, kJSmem, s>>>(0, w.nkeep, nullptr, w.C, kMaxU, w.T, w.Z, kMaxU,
-                                                    kSchurSweeps, kSchurTol, w.sweeps);
+                                                    kSchurSweeps, kSchurTol, w.sweeps, w.log);
+    QD_CHECK_LAUNCH();
+    cap_schur_z_kernel<<<u, kZThreads, 0, s>>>(0, w.nkeep, nullptr, w.sweeps, w.log, w.Z, kMaxU);
     QD_CHECK_LAUNCH();
     cap_select_kernel<<<1, kMaxU, 0, s>>>(w.nkeep, b, w.T, w.sel, w.theta, w.status);
     QD_CHECK_LAUNCH();
@@ -1540,16 +1610,31 @@ extern "C" int qd_complex_schur(int n, const void *d_C, int ldc, void *d_T, void
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   QD_CUDA_TRY(smem_opt_in<cap_schur_kernel>(kJSmem));
   int *d_sw = nullptr;
+  double2 *d_log = nullptr;    // beyond kSchurSweeps the kernel rotates Z itself
   QD_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(&d_sw), 2 * sizeof(int), s));
+  if (max_sweeps <= kSchurSweeps) {
+    const cudaError_t me = cudaMallocAsync(reinterpret_cast<void **>(&d_log), kSchurLog * sizeof(double2), s);
+    if (me != cudaSuccess) {
+      cudaGetLastError();
+      d_log = nullptr;
+    }
+  }
   cap_schur_kernel<<<kJC, kJThreads, kJSmem, s>>>(n, nullptr, nullptr, static_cast<const double2 *>(d_C),
                                                   ldc, static_cast<double2 *>(d_T),
                                                   static_cast<double2 *>(d_Z), ldt, max_sweeps,
-                                                  kSchurTol, d_sw);
+                                                  kSchurTol, d_sw, d_log);
   cudaError_t e = cudaGetLastError();
   QD_LAUNCHED();
+  if (e == cudaSuccess && d_log) {
+    cap_schur_z_kernel<<<n, kZThreads, 0, s>>>(n, nullptr, nullptr, d_sw, d_log,
+                                               static_cast<double2 *>(d_Z), ldt);
+    e = cudaGetLastError();
+    QD_LAUNCHED();
+  }
   int sw[2] = {0, 0};
   if (e == cudaSuccess) e = cudaMemcpyAsync(sw, d_sw, 2 * sizeof(int), cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(d_sw, s);
+  if (d_log) cudaFreeAsync(d_log, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return QD_ERR_CUDA;
   if (h_sweeps) *h_sweeps = sw[0];
