@@ -8,7 +8,7 @@
 // 139-238, a stub in the reference build).
 //
 // Layout: all dots' rows are concatenated; every vector block is row-major
-// (n_total x B).  Rows are cut into chunks of kChunkRows rows that never span
+// (n_total x B).  Rows are cut into chunks of chunk_rows_of() rows that never span
 // two dots; every row-parallel kernel runs one CTA per chunk and returns at
 // once for a dot that has converged, so one launch serves the whole batch and
 // the work of uneven dots is balanced by the hardware scheduler.
@@ -52,13 +52,16 @@
 
 namespace {
 
-constexpr int kChunkRows = 1024;      // default rows per chunk (qd_lobpcg_opts.chunk_rows)
-
 // Rows per chunk (the CTA unit of every row-parallel kernel): the option's
-// value when it is a multiple of 64 in [256, 8192], else the default.
-int chunk_rows_of(const qd_lobpcg_opts *opts) {
+// value when it is a multiple of 64 in [256, 8192], else by the batch's rows, so
+// that small batches have enough CTAs and large ones few partial sums.  Whole
+// solves at 1024 / 512 / 256 / 128 rows per chunk: 4.9k rows 9.9 / 9.7 / 9.4 /
+// 8.6 ms, 19k rows - / 17.1 / 16.9 / 13.9, 59k rows - / 27.1 / 28.8 / 32.8, 188k rows
+// 27.3 / 26.3 / 24.7 / 28.0, 473k rows 51.6 / 49.8 / 55.8 / 72.3.
+int chunk_rows_of(const qd_lobpcg_opts *opts, int64_t n_rows) {
   const int c = opts ? opts->chunk_rows : 0;
-  return (c >= 256 && c <= 8192 && c % 64 == 0) ? c : kChunkRows;
+  if (c >= 256 && c <= 8192 && c % 64 == 0) return c;
+  return n_rows <= 32768 ? 128 : n_rows <= 300000 ? 512 : 1024;
 }
 constexpr int kMaxB = 16;
 constexpr int kMaxM = 3 * kMaxB;
@@ -2995,7 +2998,7 @@ int solve_b(int32_t n_dots, const int32_t *h_row_off, const int32_t *d_rowptr,
             double *d_res_out, int32_t *d_iters_out, int32_t *h_info, int32_t *h_counts,
             void *d_work, size_t work_bytes, const qd_lobpcg_opts *opts, cudaStream_t s) {
   const int64_t n_rows = h_row_off[n_dots];
-  const int chunk_rows = chunk_rows_of(opts);
+  const int chunk_rows = chunk_rows_of(opts, n_rows);
   const int nchunks = count_chunks(n_dots, h_row_off, chunk_rows);
   int64_t ntx = 0, nty = 0;
   if (h_prec) {
@@ -3238,12 +3241,13 @@ extern "C" int qd_lobpcg_workspace_size(int32_t n_dots, int64_t n_rows_total,
       b % 4)
     return QD_ERR_INVALID;
   // upper bound on the chunk count: every dot contributes at most one partial chunk
-  const int nchunks = int(n_rows_total / chunk_rows_of(opts)) + n_dots;
+  const int chunk_rows = chunk_rows_of(opts, n_rows_total);
+  const int nchunks = int(n_rows_total / chunk_rows) + n_dots;
   int64_t ntx = 0, nty = 0;
   if (h_prec) qd::dst_tiles(n_dots, h_prec, b, nullptr, &ntx, nullptr, &nty);
   qd::Arena ar(nullptr, 0);
   Layout L;
-  carve(ar, n_dots, n_rows_total, nnz_total, b, nchunks, chunk_rows_of(opts), ntx, nty,
+  carve(ar, n_dots, n_rows_total, nnz_total, b, nchunks, chunk_rows, ntx, nty,
         prec_mode == QD_PREC_MIXED, needs_jacobi(n_dots, h_prec), L);
   *bytes = ar.used;
   return QD_OK;
