@@ -176,7 +176,7 @@ typedef struct {
  *   tol32        estimate at which a dot leaves the FP32 phase (<= 0: max(100 tol, 1e-7))
  *   stag_window  FP32 iterations without halving the estimate before a dot
  *                switches to FP64 anyway (<= 0: 12)
- *   graphs       nonzero: replay blocks of 8 iterations as one CUDA graph
+ *   graphs       nonzero: run the iterations as one CUDA graph loop
  *                (default); 0: enqueue every kernel directly
  *   x0           optional device array (rows x k, the layout of d_X_out): warm
  *                start for the first k block vectors (e.g. the previous

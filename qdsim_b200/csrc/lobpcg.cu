@@ -2810,7 +2810,7 @@ int run_solver(const Layout &L, bool mixed, int n_dots, const int32_t *rowptr, c
     }
     return QD_OK;
   };
-  // Iterations run in blocks of kGraphBlock.  The first block is enqueued
+  // Iterations run in blocks.  The first block is enqueued
   // directly (it also sets every kernel's attributes).  The rest of the solve
   // is one CUDA graph: a WHILE conditional node whose body is one block of
   // iterations followed by loop_control_kernel, which counts the active dots
@@ -2823,9 +2823,14 @@ int run_solver(const Layout &L, bool mixed, int n_dots, const int32_t *rowptr, c
   // unavailable, with per-kernel timing enabled, or with graphs switched off
   // in the options, blocks are enqueued directly and the host reads the
   // active-dot count after each one.
-  constexpr int kGraphBlock = 8;
+  // A block of the device loop is two iterations: the last block runs past the
+  // slowest dot's convergence (empty launches), and the graph is instantiated
+  // on every call (P1 dot of 4.9k rows 8.5 ms at eight, 8.1 at four, 7.8 at
+  // two; 64 P2 dots 87.1, 86.3, 86.0 ms).  Without it a block ends in a read by the
+  // host: eight.
   const bool graphs = use_graphs && !qd::prof_enabled();
-  const int total_blocks = (prm.max_iter + kGraphBlock + kGraphBlock - 1) / kGraphBlock;
+  const int block = graphs ? 2 : 8;
+  const int total_blocks = (prm.max_iter + block + block - 1) / block;
   struct GraphGuard {
     cudaStream_t cap = nullptr;
     cudaGraph_t graph = nullptr;
@@ -2837,15 +2842,15 @@ int run_solver(const Layout &L, bool mixed, int n_dots, const int32_t *rowptr, c
     }
   } gg;
   iters_run = 0;
-  for (int i = 0; i < kGraphBlock; ++i) {
+  for (int i = 0; i < block; ++i) {
     const int st = iteration(s);
     if (st != QD_OK) return st;
   }
-  iters_run = kGraphBlock;
+  iters_run = block;
   if (total_blocks <= 1) return QD_OK;
   bool device_loop = false;
   if (graphs) {
-    // WHILE graph: [check] -> WHILE(cond) { kGraphBlock iterations; control }
+    // WHILE graph: [check] -> WHILE(cond) { block iterations; control }
     cudaGraphConditionalHandle cond;
     cudaGraphNode_t pre = nullptr, loop = nullptr;
     size_t nnodes = 1;
@@ -2879,7 +2884,7 @@ int run_solver(const Layout &L, bool mixed, int n_dots, const int32_t *rowptr, c
                                                   cudaStreamCaptureModeThreadLocal));
         const uint64_t l0 = qd::g_launches.load();
         int st = QD_OK;
-        for (int i = 0; i < kGraphBlock && st == QD_OK; ++i) st = iteration(gg.cap);
+        for (int i = 0; i < block && st == QD_OK; ++i) st = iteration(gg.cap);
         if (st == QD_OK) {
           loop_control_kernel<<<1, 256, 0, gg.cap>>>(L.st, n_dots, L.count, total_blocks - 1,
                                                      L.wait_err, cond, 0);
@@ -2901,7 +2906,7 @@ int run_solver(const Layout &L, bool mixed, int n_dots, const int32_t *rowptr, c
           qd::g_launches.fetch_add(body_launches * uint64_t(blocks - 1),
                                    std::memory_order_relaxed);
         if (blocks == 0) qd::g_launches.fetch_sub(body_launches, std::memory_order_relaxed);
-        iters_run += kGraphBlock * blocks;
+        iters_run += block * blocks;
         device_loop = true;
       }
     }
@@ -2915,11 +2920,11 @@ int run_solver(const Layout &L, bool mixed, int n_dots, const int32_t *rowptr, c
       QD_CUDA_TRY(cudaMemcpyAsync(&host_count, L.count, sizeof(int), cudaMemcpyDeviceToHost, s));
       QD_CUDA_TRY(cudaStreamSynchronize(s));
       if (host_count == 0) break;
-      for (int i = 0; i < kGraphBlock; ++i) {
+      for (int i = 0; i < block; ++i) {
         const int st = iteration(s);
         if (st != QD_OK) return st;
       }
-      iters_run += kGraphBlock;
+      iters_run += block;
     }
   }
   return QD_OK;
