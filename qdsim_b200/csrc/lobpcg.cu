@@ -1152,10 +1152,10 @@ __device__ __forceinline__ bool chol_congruence(Tile<TM> &Bm, Tile<TM> &A, Tile<
 //   (3) inverse iteration on T - lambda_j I (Gaussian elimination with row
 //       interchanges, factored once; a back-substitution from a fixed
 //       pseudo-random vector, then one full step), one thread per
-//       eigenvalue, then classical Gram-Schmidt over the nsel vectors in
-//       ascending order, repeated for a vector that was not yet orthogonal to
-//       1e-6 (inside clusters of close eigenvalues, which inverse iteration
-//       alone does not separate);
+//       eigenvalue, then one step of symmetric orthonormalisation, or, inside
+//       clusters of close eigenvalues, which inverse iteration alone does not
+//       separate, classical Gram-Schmidt over the nsel vectors in ascending
+//       order, repeated for a vector that was not yet orthogonal to 1e-6;
 //   (4) back-transformation Z = H Y, 16 lanes per vector, in registers.
 // Eigenvalues ascending into ev[0..nsel), eigenvectors into Z's columns
 // 0..nsel-1 (ldz).  work: 4 n nsel doubles; Vs: n x 16 TM doubles; sw: 10 * 16 TM
@@ -1203,15 +1203,23 @@ __device__ __forceinline__ void tridiag_lowest_cta(Tile<TM> &A, double *Z, int l
 #pragma unroll
       for (int a = 0; a < TM; ++a) y[a] = fma(A.v[a][b], xc[b], y[a]);
     }
-#pragma unroll
-    for (int o = 8; o; o >>= 1) {
-      s2 += __shfl_xor_sync(ALL, s2, o);
-#pragma unroll
-      for (int a = 0; a < TM; ++a) y[a] += __shfl_xor_sync(ALL, y[a], o);
-    }
-    if (tx == 0) {
-#pragma unroll
-      for (int a = 0; a < TM; ++a) ys[ty + 16 * a] = y[a];
+    // sums over the 16 lanes of tx: each exchange halves the values a lane keeps,
+    // which ends with y_0, y_1, y_2, |x|^2 on lanes 0, 4, 8, 12
+    {
+      const bool h8 = tx & 8, h4 = tx & 4;
+      const double y1 = TM > 1 ? y[TM > 1 ? 1 : 0] : 0.0, y2 = TM > 2 ? y[TM > 2 ? 2 : 0] : 0.0;
+      double u = h8 ? y2 : y[0], w = h8 ? s2 : y1;
+      u += __shfl_xor_sync(ALL, h8 ? y[0] : y2, 8);
+      w += __shfl_xor_sync(ALL, h8 ? y1 : s2, 8);
+      double c = h4 ? w : u;
+      c += __shfl_xor_sync(ALL, h4 ? u : w, 4);
+      c += __shfl_xor_sync(ALL, c, 2);
+      c += __shfl_xor_sync(ALL, c, 1);
+      if ((tx & 3) == 0) {
+        const int q = tx >> 2;
+        if (q < TM) ys[ty + 16 * q] = c;
+        if (q == 3 && ty == 0) sdt[0] = c;
+      }
     }
     if (tx == ((k + 1) & 15)) {
 #pragma unroll
@@ -1219,7 +1227,7 @@ __device__ __forceinline__ void tridiag_lowest_cta(Tile<TM> &A, double *Z, int l
     }
     __syncthreads();
     const double x0 = x[k + 1];
-    // |x|^2 is the same sum in every thread, and so is this test
+    s2 = sdt[0];
     if (s2 - x0 * x0 <= 1e-300 * fmax(1.0, s2)) {   // column already reduced
       if (tid == 0) {
         se[k] = x0;
@@ -1333,6 +1341,7 @@ __device__ __forceinline__ void tridiag_lowest_cta(Tile<TM> &A, double *Z, int l
   }
   __syncthreads();
   // (3)
+  int gs_from = 1;
   if (tid < nsel) {
     const int j = tid, W = nsel;
     double *di = work, *su = work + n * W, *su2 = work + 2 * n * W, *ml = work + 3 * n * W;
@@ -1386,13 +1395,44 @@ __device__ __forceinline__ void tridiag_lowest_cta(Tile<TM> &A, double *Z, int l
       }
       scale = rsqrt(fmax(nrm, 1e-300));
     }
-    for (int i = 0; i < n; ++i) Z[i * ldz + j] *= scale;
     ev[j] = lam * up;
   }
   __syncthreads();
-  // classical Gram-Schmidt in ascending order: warp w forms the coefficients
-  // against vectors i = w, w + 8, ..., all threads subtract, warp 0 normalises
-  for (int j = 1; j < nsel; ++j) {
+  // Orthonormalisation.  The vectors of well separated eigenvalues are orthogonal
+  // to far below 1e-9 already: with G = D^-1/2 Z^T Z D^-1/2 = I + E one step
+  // Z D^-1/2 (I - E / 2) leaves |E|^2.
+  {
+    double *sG = work, *sn = sdt;                  // [nsel][nsel], [16]
+    double g = 0.0;
+    if (ty < nsel && tx < nsel)
+      for (int r = 0; r < n; ++r) g = fma(Z[r * ldz + ty], Z[r * ldz + tx], g);
+    if (ty == tx) sn[tx] = rsqrt(fmax(g, 1e-300));
+    __syncthreads();
+    const double e = ty < nsel && tx < nsel ? (ty == tx ? 0.0 : g * sn[ty] * sn[tx]) : 0.0;
+    if (ty < nsel && tx < nsel) sG[ty * nsel + tx] = -0.5 * e;
+    const bool apart = __syncthreads_or(!(fabs(e) <= 1e-9)) == 0;
+    double z[TM];
+#pragma unroll
+    for (int a = 0; a < TM; ++a) {
+      const int r = ty + 16 * a;
+      z[a] = 0.0;
+      if (r < n && tx < nsel) {
+        z[a] = Z[r * ldz + tx] * sn[tx];
+        if (apart)
+          for (int i = 0; i < nsel; ++i) z[a] = fma(Z[r * ldz + i] * sn[i], sG[i * nsel + tx], z[a]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < TM; ++a)
+      if (ty + 16 * a < n && tx < nsel) Z[(ty + 16 * a) * ldz + tx] = z[a];
+    __syncthreads();
+    gs_from = apart ? nsel : 1;
+  }
+  // otherwise classical Gram-Schmidt in ascending order: warp w forms the
+  // coefficients against vectors i = w, w + 8, ..., all threads subtract, warp 0
+  // normalises
+  for (int j = gs_from; j < nsel; ++j) {
     for (int pass = 0; pass < 2; ++pass) {
       for (int i = warp; i < j; i += nt / 32) {
         double dt = 0.0;
@@ -1462,9 +1502,9 @@ __device__ __forceinline__ void tridiag_lowest_cta(Tile<TM> &A, double *Z, int l
 // chains of small dependent steps and the barriers between them (about seven
 // cycles per instruction and warp).  With the matrices in registers, the
 // congruence in place of two triangular products, and bisection without
-// divisions it takes about 165 us at B = 16 and 130 us at B = 12 where the form
-// in shared memory took 377 and 220 us (and 500 us with SVQB in every step of the
-// plain FP64 form, which now takes it only when a pivot is small).
+// divisions a launch takes 132 us at B = 16 (64 dots) and 97 us at B = 12 where
+// the form in shared memory took 377 and 201 us (499 us with SVQB in every step
+// of the plain FP64 form, which now takes it only when a pivot is small).
 template <int B>
 __global__ void __launch_bounds__(256)
 rr_kernel(DotState *st, const double *partial, const double *norms, double *theta,
