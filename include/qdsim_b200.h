@@ -527,6 +527,14 @@ int qd_adjoint(int order, int64_t num_nodes, int64_t num_elems, int n_states, in
                const int32_t *d_nadjptr, const int32_t *d_nadj,
                double *d_dLdV, double *d_dLdc, double *d_work, void *stream);
 
+/* qd_adjoint with the weights in host memory (read before the call returns, so
+ * that no copy to the device stands in front of the launch). */
+int qd_adjoint_host_weights(int order, int64_t num_nodes, int64_t num_elems, int n_states,
+                            int is_complex, const double *d_nodes, const int32_t *d_elems,
+                            const int32_t *d_dofmap, const double *d_psi, const double *h_w,
+                            const int32_t *d_nadjptr, const int32_t *d_nadj, double *d_dLdV,
+                            double *d_dLdc, double *d_work, void *stream);
+
 /* ---------------------------------------------------------------------------
  * Per-kernel-kind timing with CUDA events, recorded on the stream of each
  * launch (off by default).  Kinds: 0 SpMM, 1 Gram, 2 Rayleigh-Ritz, 3 update,

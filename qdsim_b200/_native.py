@@ -82,6 +82,8 @@ SIGNATURES = {
     "qd_sc_mix": (_int, [_i32, _i64, _int, _int, _p, _p, _p, _p, _p, _p, _p, _p, _p]),
     "qd_adjoint": (_int, [_int, _i64, _i64, _int, _int, _p, _p, _p, _p, _p, _p, _p,
                           _p, _p, _p, _p]),
+    "qd_adjoint_host_weights": (_int, [_int, _i64, _i64, _int, _int, _p, _p, _p, _p, _p, _p, _p,
+                                       _p, _p, _p, _p]),
     "qd_cap_lobpcg_workspace_size": (_int, [_i32, _int, _int, _p, _p]),
     "qd_cap_lobpcg_solve": (_int, [_i32, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _int, _int, _int,
                                    _dbl, _dbl, _dbl, _int, _int, _dbl, _u64, _p, _p, _p, _p, _p,

@@ -123,8 +123,9 @@ def energy_gradients(prob: FEMProblem, psi_reduced: torch.Tensor, weights, strea
     else:
         if np.iscomplexobj(w) and np.any(np.imag(w) != 0):
             raise ValueError("complex weights need complex eigenvectors")
-        wv = np.real(w).astype(np.float64)
-    wt = torch.as_tensor(wv, dtype=torch.float64, device=dev)
+        wv = np.ascontiguousarray(np.real(w), dtype=np.float64).reshape(-1)
+    if wv.size < (2 if cplx else 1) * ns:
+        raise ValueError("one weight per state")
     nptr, nadj = prob.node_adjacency()
     m = prob.mesh
     if not hasattr(prob, "_adj_out"):
@@ -132,10 +133,11 @@ def energy_gradients(prob: FEMProblem, psi_reduced: torch.Tensor, weights, strea
     dV, dc, work = prob._adj_out.get(m, dev)
     if out is not None:
         dV, dc = out
-    N.check(N.lib().qd_adjoint(m.order, m.num_nodes, m.num_elements, ns, 1 if cplx else 0,
-                               N.ptr(prob.d_nodes), N.ptr(prob.d_elems), N.ptr(prob.d_dofmap),
-                               N.ptr(psi), N.ptr(wt), N.ptr(nptr), N.ptr(nadj), N.ptr(dV),
-                               N.ptr(dc), N.ptr(work), stream_ptr(stream)), "qd_adjoint")
+    N.check(N.lib().qd_adjoint_host_weights(
+        m.order, m.num_nodes, m.num_elements, ns, 1 if cplx else 0, N.ptr(prob.d_nodes),
+        N.ptr(prob.d_elems), N.ptr(prob.d_dofmap), N.ptr(psi), N.ptr(wv), N.ptr(nptr),
+        N.ptr(nadj), N.ptr(dV), N.ptr(dc), N.ptr(work), stream_ptr(stream)),
+        "qd_adjoint_host_weights")
     return dV, dc
 
 
