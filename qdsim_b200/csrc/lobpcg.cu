@@ -728,16 +728,17 @@ cudaError_t smem_attr(size_t bytes) {
   return e;
 }
 
-// Gram tasks: one upper-triangle 4x4 block (bi <= bj) of S^T HS or of S^T MS
-// per thread (NT2 = 2 NT tasks), RG row groups.  One matrix per thread keeps
-// the FP64 accumulators at 16 values, so two CTAs fit on an SM.
+// Gram tasks: one upper-triangle 4x4 block (bi <= bj) per thread, RG row groups.
+// FP32: of S^T HS and of S^T MS both (NM = 2), so that the four values of S are
+// read once for both; FP64: of one of the two (NM = 1: 16 FP64 accumulators, so
+// that two CTAs fit on an SM).
 template <typename TV, int B> struct GramCfg {
   static constexpr int m = 3 * B;
   static constexpr int NB = m / 4;
   static constexpr int NT = NB * (NB + 1) / 2;            // upper-triangle 4x4 blocks
-  static constexpr int NT2 = 2 * NT;                      // of S^T HS, then of S^T MS
-  static constexpr int TARGET = sizeof(TV) == 8 ? 256 : 384;
-  static constexpr int RG = (TARGET / NT2) > 0 ? (TARGET / NT2) : 1;
+  static constexpr int NM = sizeof(TV) == 8 ? 1 : 2;
+  static constexpr int NT2 = NM == 2 ? NT : 2 * NT;       // tasks
+  static constexpr int RG = (256 / NT2) > 16 ? 16 : ((256 / NT2) > 0 ? (256 / NT2) : 1);
   static constexpr int THREADS = ((NT2 * RG + 31) / 32) * 32;
 };
 
@@ -764,13 +765,124 @@ template <> __device__ inline void lds4<double>(const double *p, double (&v)[4])
   v[3] = b.y;
 }
 
-template <typename TV, int B> using GramPipe = qd::BlockPipe<TV, B, 9, (sizeof(TV) == 8 ? 32 : 64), 3>;
+template <typename TV, int B>
+using GramPipe = qd::BlockPipe<TV, B, 9, sizeof(TV) == 8 ? 32 : (B == 12 ? 80 : 64), 3>;
 
+// The 4x4 outer products of one row for a task, added to t[NM][4][4].  FP32: in
+// pairs (fma.rn.f32x2, each half rounded as a single fma): (a0, a1) times
+// (b0, b1) and times the swapped (a1, a0) gives all four products of the pairs,
+// so only the two pairs of S are swapped, once for both matrices.
+struct GramAcc64 {
+  double t[16];
+  __device__ void zero() {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) t[q] = 0.0;
+  }
+  __device__ void add(const double *s, const double *r, int) {
+    double sa[4], rb[4];
+    lds4(s, sa);
+    lds4(r, rb);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) t[4 * a + b] = fma(sa[a], rb[b], t[4 * a + b]);
+  }
+  __device__ void flush(double *acc) const {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) acc[q] += t[q];
+  }
+};
+struct GramAcc32 {
+  // t[w][p][q][x]: pairs p of S, q of R; x = 0: (a0 b0, a1 b1), 1: (a1 b0, a0 b1)
+  unsigned long long t[2][2][2][2];
+  __device__ void zero() {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) (&t[0][0][0][0])[q] = 0ull;
+  }
+  __device__ void add(const float *s, const float *r, int stride) {
+    const ulonglong2 sv = *reinterpret_cast<const ulonglong2 *>(s);
+    const unsigned long long sp[2] = {sv.x, sv.y};
+    unsigned long long sx[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+      asm("{ .reg .b32 lo, hi;\n mov.b64 {lo, hi}, %1;\n mov.b64 %0, {hi, lo}; }"
+          : "=l"(sx[p]) : "l"(sp[p]));
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const ulonglong2 rv = *reinterpret_cast<const ulonglong2 *>(r + w * stride);
+      const unsigned long long rp[2] = {rv.x, rv.y};
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(t[w][p][q][0]) : "l"(sp[p]), "l"(rp[q]));
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(t[w][p][q][1]) : "l"(sx[p]), "l"(rp[q]));
+        }
+    }
+  }
+  __device__ void flush(double *acc) const {
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const float lo = __uint_as_float(unsigned(t[w][p][q][x]));
+            const float hi = __uint_as_float(unsigned(t[w][p][q][x] >> 32));
+            acc[16 * w + 4 * (2 * p + x) + 2 * q] += double(lo);
+            acc[16 * w + 4 * (2 * p + 1 - x) + 2 * q + 1] += double(hi);
+          }
+  }
+};
+
+// task -> its 4-column groups bi <= bj of S.  B = 16: the triangles of (X, X),
+// (W, W), (P, P), then (X, W), (X, P), (W, P) row by row, so that the eight
+// lanes that a 16-byte shared load serves at once read few and neighbouring
+// groups (X and P rows fall on the same banks; row order over the whole triangle
+// takes 26 % more wavefronts).  Otherwise row order: the 3 B / 4 groups of a row
+// lie side by side on the banks (at B = 12 the blocked order takes 6 % more).
+template <int B>
+__device__ inline void gram_task(int task, int &bi, int &bj) {
+  constexpr int G = B / 4, TRI = G * (G + 1) / 2;
+  if constexpr (B != 16) {
+    int a = 0;
+    while (task >= 3 * G - a) {
+      task -= 3 * G - a;
+      ++a;
+    }
+    bi = a;
+    bj = a + task;
+    return;
+  }
+  if (task < 3 * TRI) {
+    const int blk = task / TRI;
+    int a = 0, rem = task % TRI;
+    while (rem >= G - a) {
+      rem -= G - a;
+      ++a;
+    }
+    bi = blk * G + a;
+    bj = bi + rem;
+  } else {
+    const int u = task - 3 * TRI, blk = u / (G * G), r = u % (G * G);
+    bi = (blk == 2 ? G : 0) + r / G;
+    bj = (blk == 0 ? G : 2 * G) + r % G;
+  }
+}
+
+// Bound in FP32 by the issue of 16-byte shared loads (four wavefronts each, 60 %
+// of the pipe) and the latency behind them, not by HBM (64 % of it): per row a
+// task reads 48 bytes for 32 products.  All 64 dots iterating, B = 12, 2.45 M
+// rows: 345 us with one matrix per thread, 274 us with both, pairs of products
+// and sub-tiles of 80 rows (16 per row group, as many as FP32 summed before);
+// B = 16, 1.91 M rows: 426 us before, 329 us now.
 // Each thread owns one upper-triangle 4x4 block (bi <= bj) of both S^T HS and
-// S^T MS for a slice (row group rg) of every sub-tile's rows, accumulating
-// in TV within a sub-tile and in FP64 across sub-tiles.  Off-diagonal blocks
-// are written to both (bi, bj) and (bj, bi), so the per-chunk partial holds
-// the full symmetric matrices.
+// S^T MS (FP32) or of one of them (FP64) for a slice (row group rg) of every
+// sub-tile's rows, accumulating in TV within a sub-tile and in FP64 across
+// sub-tiles.  Off-diagonal blocks are written to both (bi, bj) and (bj, bi), so
+// the per-chunk partial holds the full symmetric matrices.
 template <typename TV, int B>
 __global__ void __launch_bounds__(GramCfg<TV, B>::THREADS, 2)
 gram_kernel(const Chunk *chunks, const DotState *st, const TV *X, const TV *W, const TV *P,
@@ -778,8 +890,10 @@ gram_kernel(const Chunk *chunks, const DotState *st, const TV *X, const TV *W, c
             double *partial, int *wait_err) {
   using C = GramCfg<TV, B>;
   using PP = GramPipe<TV, B>;
-  constexpr int m = C::m, NB = C::NB, NT = C::NT, NT2 = C::NT2, RG = C::RG;
+  constexpr int m = C::m, NB = C::NB, NT = C::NT, NT2 = C::NT2, RG = C::RG, NM = C::NM;
   constexpr int BLK = PP::BLKP;   // block stride inside a stage
+  constexpr int NA = 16 * NM;
+  using Acc = typename std::conditional<sizeof(TV) == 8, GramAcc64, GramAcc32>::type;
   extern __shared__ __align__(128) unsigned char dsm[];
 
   const Chunk ch = chunks[blockIdx.x];
@@ -789,23 +903,16 @@ gram_kernel(const Chunk *chunks, const DotState *st, const TV *X, const TV *W, c
     const_cast<DotState *>(st)[ch.dot].launches[sizeof(TV) == 8][1]++;
   const bool worker = tid < NT2 * RG;
   const int task2 = tid % NT2, rg = tid / NT2;
-  const int which = task2 / NT, task = task2 % NT;   // which: 0 S^T HS, 1 S^T MS
-  // task -> (bi, bj) with bi <= bj
-  int bi = 0, rem = task;
-  while (rem >= NB - bi) {
-    rem -= NB - bi;
-    ++bi;
-  }
-  const int bj = bi + rem;
+  const int which = task2 / NT, task = task2 % NT;   // NM == 1: 0 S^T HS, 1 S^T MS
+  int bi, bj;
+  gram_task<B>(task, bi, bj);
   // element offsets of this thread's 4 columns inside a stage (B % 4 == 0,
   // so a group of 4 columns never straddles two blocks)
   const int offS = ((4 * bi) / B) * BLK + (4 * bi) % B;
   const int offR = (3 + 3 * which + (4 * bj) / B) * BLK + (4 * bj) % B;
-  double acc[4][4];
+  double acc[NA];                 // [matrix][a][b]
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+  for (int q = 0; q < NA; ++q) acc[q] = 0.0;
 
   const TV *src[9] = {X, W, P, HX, HW, HP, MX, MW, MP};
   PP pipe;
@@ -816,58 +923,47 @@ gram_kernel(const Chunk *chunks, const DotState *st, const TV *X, const TV *W, c
     if (worker && ok) {
       const int nr = pipe.rows(i);
       const TV *sb = pipe.tile(i, 0);
-      TV t[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) t[a][b] = TV(0);
-      for (int row = rg; row < nr; row += RG) {
-        TV sa[4], rb[4];
-        lds4(sb + offS + row * B, sa);
-        lds4(sb + offR + row * B, rb);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) t[a][b] = fma(sa[a], rb[b], t[a][b]);
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] += double(t[a][b]);
+      Acc t;
+      t.zero();
+#pragma unroll 2
+      for (int row = rg; row < nr; row += RG)
+        t.add(sb + offS + row * B, sb + offR + row * B, 3 * BLK);
+      t.flush(acc);
     }
     pipe.release(i, ok);
   }
   if (!pipe.finish(ok, wait_err)) return;
   double *out = partial + size_t(blockIdx.x) * 2 * m * m;
   if (RG > 1) {
-    double *red = reinterpret_cast<double *>(dsm);   // NT2 * 16 doubles < one stage
+    double *red = reinterpret_cast<double *>(dsm);   // NT2 * NA doubles < one stage
+    static_assert(NT2 * NA * sizeof(double) <= PP::BAR_OFF, "reduction slots");
     for (int g = 1; g < RG; ++g) {
       if (worker && rg == g) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) red[task2 * 16 + a * 4 + b] = acc[a][b];
+        for (int q = 0; q < NA; ++q) red[q * NT2 + task2] = acc[q];
       }
       __syncthreads();
       if (worker && rg == 0) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] += red[task2 * 16 + a * 4 + b];
+        for (int q = 0; q < NA; ++q) acc[q] += red[q * NT2 + task2];
       }
       __syncthreads();
     }
   }
   if (worker && rg == 0) {
-    double *o = out + size_t(which) * m * m;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int w = 0; w < NM; ++w) {
+      double *o = out + size_t(which + w) * m * m;
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int i = 4 * bi + a, j = 4 * bj + b;
-        o[i * m + j] = acc[a][b];
-        if (bi != bj) o[j * m + i] = acc[a][b];
-      }
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int i = 4 * bi + a, j = 4 * bj + b;
+          const double v = acc[16 * w + 4 * a + b];
+          o[i * m + j] = v;
+          if (bi != bj) o[j * m + i] = v;
+        }
+    }
   }
 }
 
