@@ -72,6 +72,8 @@ class CAPProblem:
         self.n = self.fem.n
         spec = DSTPreconditioner.spec_for(mesh, c_elem, V, shift_ev)
         self.prec = DSTPreconditioner([spec], self.device) if spec is not None else None
+        # free rows per lattice row (the products' row order), 0 without a lattice
+        self._width = int(self.prec.desc[0]["nx"]) if self.prec is not None else 0
         self._pws = None
         self._work = None
 
@@ -92,9 +94,8 @@ class CAPProblem:
             if T.stride(1) != 1 or T.shape[0] != self.n:
                 raise ValueError("cap spmm operands must be [n, b] with unit column stride")
         H, G, M = (self.H32, self.G32, self.M32) if fp32 else (self.H, self.G, self.M)
-        width = int(self.prec.desc[0]["nx"]) if self.prec is not None else 0
         N.check(N.lib().qd_cap_spmm_lattice(
-            self.n, width, b, 1 if fp32 else 0, N.ptr(self.fem.d_rowptr), N.ptr(self.fem.d_col),
+            self.n, self._width, b, 1 if fp32 else 0, N.ptr(self.fem.d_rowptr), N.ptr(self.fem.d_col),
             N.ptr(H), N.ptr(G), N.ptr(M), N.ptr(X), X.stride(0), N.ptr(AX), N.ptr(MX),
             AX.stride(0), stream_ptr()), "qd_cap_spmm_lattice")
 
