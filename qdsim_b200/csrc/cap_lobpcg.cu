@@ -700,7 +700,9 @@ cap_schur_kernel(int n_fix, const int *__restrict__ n_dev, const int *__restrict
 #pragma unroll
   for (int o = 16; o; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
   if (lane == 0) s_w[warp] = nrm;
-  __syncthreads();
+  // a CTA's shared memory may be written by another only once it has started, so
+  // the whole cluster meets here, before the first store to a peer
+  cluster.sync();
   if (tid == 0) {
     double sacc = 0.0;
     for (int w = 0; w < kJThreads / 32; ++w) sacc += s_w[w];
