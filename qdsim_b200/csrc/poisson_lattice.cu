@@ -49,6 +49,13 @@ constexpr int kMT = 64;            // modes (rows) per transform tile
 constexpr int kKC = 16;            // contraction depth per stage
 constexpr int kAP = kKC + 4, kBP = kNT + 4;   // pitches: fragments without bank conflicts
 constexpr int kSweepT = 128;
+// shared memory of a sweep block with cw columns: a line's factors and values
+__host__ __device__ constexpr size_t sweep_bytes(int nx, int cw) {
+  return size_t(nx + 1) * (sizeof(double2) + 8 * size_t(cw));
+}
+constexpr size_t kSweepWide = size_t(100) << 10;              // most for cw > 1
+constexpr size_t kSweepMax = sweep_bytes(kMaxNx, 1);          // most of all: one column
+static_assert(kSweepMax >= kSweepWide && kSweepMax <= (size_t(227) << 10), "fits an SM");
 
 struct Dims {
   int nx, ny, nrhs, n;    // n = (nx + 1)(ny + 1)
@@ -651,15 +658,16 @@ extern "C" int qd_poisson_lattice_solve(int nx, int ny, int nrhs, const int32_t 
   const dim3 cgrid((d.Q + kNT - 1) / kNT, d.Hp / kMT);
   const int cbytes = 2 * int(sizeof(Stage));
   int cw = std::min(32, nrhs);
-  auto sweep_bytes = [&](int c) { return size_t(nx + 1) * (sizeof(double2) + 8 * size_t(c)); };
-  while (cw > 1 && sweep_bytes(cw) > (size_t(100) << 10)) cw = (cw + 1) / 2;
+  while (cw > 1 && sweep_bytes(nx, cw) > kSweepWide) cw = (cw + 1) / 2;
   const dim3 sgrid(ny + 1, (nrhs + cw - 1) / cw);
   QD_CUDA_TRY(cudaFuncSetAttribute(lat_cos_kernel<true>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, cbytes));
   QD_CUDA_TRY(cudaFuncSetAttribute(lat_cos_kernel<false>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, cbytes));
+  // a constant, as for every kernel: the limit belongs to the process, and a
+  // smaller one set for a small lattice would fail another thread's launch
   QD_CUDA_TRY(cudaFuncSetAttribute(lat_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(sweep_bytes(cw))));
+                                   int(kSweepMax)));
   qd::prof_begin(qd::PK_PCG, s);
   QD_CUDA_TRY(cudaMemsetAsync(L.counter, 0, 4 * sizeof(unsigned), s));
   lat_init_kernel<<<G, T, 0, s>>>(d, d_rowptr, d_col, d_K, d_M, d_rho, alpha, ends, d_X0, d_X, L.R,
@@ -668,7 +676,7 @@ extern "C" int qd_poisson_lattice_solve(int nx, int ny, int nrhs, const int32_t 
   auto precond = [&]() -> int {
     lat_cos_kernel<true><<<cgrid, kT, cbytes, s>>>(d, plan, L.R, L.S, nullptr, nullptr, ctl);
     QD_CHECK_LAUNCH();
-    lat_sweep_kernel<<<sgrid, kSweepT, sweep_bytes(cw), s>>>(d, cw, tri, L.S, ctl);
+    lat_sweep_kernel<<<sgrid, kSweepT, sweep_bytes(nx, cw), s>>>(d, cw, tri, L.S, ctl);
     QD_CHECK_LAUNCH();
     lat_cos_kernel<false><<<cgrid, kT, cbytes, s>>>(d, plan, L.S, L.Z, L.R, L.dotq, ctl);
     QD_CHECK_LAUNCH();
