@@ -98,6 +98,8 @@ class PoissonProblem:
         g = torch.from_numpy(np.concatenate([gx, gy])).to(self.device)
         N.check(L.qd_poisson_lattice_plan(m.nx, m.ny, N.ptr(g), N.ptr(g[m.nx:]), N.ptr(plan),
                                           plan.numel(), stream_ptr()), "qd_poisson_lattice_plan")
+        # solve() may run on any stream: the plan is complete when the problem is
+        torch.cuda.current_stream().synchronize()
         return plan
 
     def rhs(self, rho):

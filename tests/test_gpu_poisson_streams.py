@@ -44,3 +44,16 @@ def test_two_threads_solve_lattices_of_unlike_sizes(cuda):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_a_new_problem_leaves_nothing_running(cuda):
+    """Whatever the constructor computes is complete when it returns, so that the
+    first solve may run on any stream.  The factors of a line of 7000 cells take
+    their one thread milliseconds."""
+    import torch
+    _problem(cuda, 7000, 4, 2)
+    assert torch.cuda.current_stream().query()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        _problem(cuda, 7000, 4, 3)
+        assert side.query()
