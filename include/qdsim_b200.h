@@ -346,7 +346,8 @@ int qd_csr_spmv(int32_t n, int nrhs, const int32_t *d_rowptr, const int32_t *d_c
  *   d_X0         start [n][nrhs] (not d_X; its values on x = 0, Lx are not
  *                read) or NULL
  *   tol          as in qd_pcg_solve; h_iters the iterations run
- * Limits: nx <= 8000, nrhs <= 256.  The call waits for the result.
+ * Limits: nx <= 8000, ny <= 16384 (the plan takes about 8 ny^2 + 16 n bytes),
+ * nrhs <= 256.  The call waits for the result.
  * ------------------------------------------------------------------------- */
 int qd_poisson_lattice_plan_size(int nx, int ny, size_t *bytes);
 int qd_poisson_lattice_plan(int nx, int ny, const double *d_gx, const double *d_gy, void *d_plan,

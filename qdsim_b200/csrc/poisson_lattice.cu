@@ -44,6 +44,7 @@ namespace {
 constexpr int kMaxRhs = 256;
 constexpr int kT = 256;            // threads of every kernel but the sweep
 constexpr int kMaxNx = 8000;       // one line of one column fits in shared memory
+constexpr int kMaxNy = 16384;      // 2.1 GB of cosine matrices
 constexpr int kNT = 64;            // lattice columns q per transform tile
 constexpr int kMT = 64;            // modes (rows) per transform tile
 constexpr int kKC = 16;            // contraction depth per stage
@@ -577,7 +578,7 @@ void carve(qd::Arena &ar, const Dims &d, Layout &L) {
 }
 
 bool valid_lattice(int nx, int ny, int nrhs) {
-  return nx >= 1 && nx <= kMaxNx && ny >= 1 && nrhs >= 1 && nrhs <= kMaxRhs &&
+  return nx >= 1 && nx <= kMaxNx && ny >= 1 && ny <= kMaxNy && nrhs >= 1 && nrhs <= kMaxRhs &&
          (int64_t(nx) + 1) * (int64_t(ny) + 1) <= INT32_MAX &&
          (int64_t(nx) + 1) * nrhs <= INT32_MAX;
 }

@@ -33,7 +33,21 @@ EPS0 = 8.854187817e-12     # qdsim_cython/solvers/poisson_solver.pyx:28
 #: two launches each).
 LATTICE_KAPPA = 64.0
 LATTICE_MAX_NX = 8000       # qd_poisson_lattice_solve's limits
+LATTICE_MAX_NY = 16384
 LATTICE_MAX_RHS = 256
+#: Bytes that the plan of any problem may take.  Its cosine matrices take 8 ny^2
+#: bytes whatever nx is: on a narrow mesh that is far more than the problem itself.
+LATTICE_PLAN_BYTES = 256 << 20
+NODE_BYTES = 200            # of a problem's mesh, pattern and matrices, about
+
+
+def lattice_fits(nx, ny):
+    """Whether an nx x ny lattice is within the separable solver's limits, and its
+    plan no larger than LATTICE_PLAN_BYTES or than the problem's other data."""
+    if nx > LATTICE_MAX_NX or ny > LATTICE_MAX_NY:
+        return False
+    nodes = (nx + 1) * (ny + 1)
+    return 8 * ny * ny + 16 * nodes <= max(LATTICE_PLAN_BYTES, NODE_BYTES * nodes)
 
 
 def lattice_means(mesh, eps):
@@ -85,7 +99,7 @@ class PoissonProblem:
         diagonal form is taken (unstructured mesh, eps varying too much along
         y, a lattice beyond the kernel's limits)."""
         m = self.mesh
-        if not isinstance(m, StructuredMesh) or m.nx > LATTICE_MAX_NX:
+        if not isinstance(m, StructuredMesh) or not lattice_fits(m.nx, m.ny):
             return None
         gx, gy, kappa = lattice_means(m, eps)
         if not kappa <= LATTICE_KAPPA:
