@@ -15,6 +15,7 @@ Units: node coordinates in nm, rho in C/m^3, phi in V.
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import numpy as np
 import torch
@@ -27,10 +28,8 @@ EPS0 = 8.854187817e-12     # qdsim_cython/solvers/poisson_solver.pyx:28
 
 
 #: Largest condition number of the separably preconditioned operator for which
-#: the lattice form is taken.  Its iterations grow with the square root of this
-#: number (about 14 sqrt(kappa) to 1e-12, at five launches each) and not with
-#: the mesh; the diagonal form's grow with the mesh width (about 3 per cell, at
-#: two launches each).
+#: the lattice form is considered.  Its iterations grow with the square root of
+#: this number and not with the mesh (lattice_pays).
 LATTICE_KAPPA = 64.0
 LATTICE_MAX_NX = 8000       # qd_poisson_lattice_solve's limits
 LATTICE_MAX_NY = 16384
@@ -48,6 +47,33 @@ def lattice_fits(nx, ny):
         return False
     nodes = (nx + 1) * (ny + 1)
     return 8 * ny * ny + 16 * nodes <= max(LATTICE_PLAN_BYTES, NODE_BYTES * nodes)
+
+
+def lattice_pays(mesh, kappa, nrhs):
+    """Whether the lattice form is the faster one, by the iterations that either
+    needs to 1e-12 and what an iteration takes (microseconds on a B200).
+
+    Lattice: 8.5 to 12.5 sqrt(kappa) iterations where eps varies at random, one or
+    two where the separable operator is the operator; five launches, a serial
+    chain over the modes and one along the line, 300 bytes a value, and dense
+    transforms at 23 TFLOP/s.  Diagonal: in proportion to nx, more on meshes that
+    are long in y or fine in y, up to 11 nx; two launches, one thread's sum over the
+    block's threads / nrhs, 88 bytes a value.  Over 278 pairs of meshes (4 x 4 to
+    1000 x 1000, nx up to 7000, ny up to 4096), eps and 1 or 64 right-hand sides, the
+    diagonal form was nowhere faster where this rule takes the lattice form.  It is
+    where the rule takes it: 8 x 4096, eps in 1..30 at random, 64 right-hand sides
+    7.8 against 85.9 ms; 8 x 512, 3.7 against 7.8 ms; 8 x 2048, one right-hand
+    side, 10.2 against 16.0 ms.  At 300 x 100 and the same eps the lattice form takes
+    12.1 ms for 64 right-hand sides where the diagonal one takes 71.8."""
+    nx, ny = mesh.nx, mesh.ny
+    hx, hy = mesh.Lx / nx, mesh.Ly / ny
+    values = (nx + 1) * (ny + 1) * nrhs
+    its = 2.0 if kappa < 1.001 else 9.0 * math.sqrt(kappa)
+    lattice = its * (42.0 + 0.145 * ny + 0.025 * nx + 6e-5 * values
+                     + 2.0 * ny * ny * (nx + 1) * nrhs / 23e6)
+    its = nx * min(11.0, 5.5 * (mesh.Ly / mesh.Lx) ** 0.3) * math.sqrt(0.5 + 0.5 * (hx / hy) ** 2)
+    diagonal = max(16.0, its) * (18.0 + 62.0 / nrhs + 1.8e-5 * values)
+    return lattice <= diagonal
 
 
 def lattice_means(mesh, eps):
@@ -97,12 +123,13 @@ class PoissonProblem:
     def _lattice_plan(self, eps):
         """Device plan of the separable preconditioner, or None where the
         diagonal form is taken (unstructured mesh, eps varying too much along
-        y, a lattice beyond the kernel's limits)."""
+        y, a lattice beyond the kernel's limits or too narrow to pay)."""
         m = self.mesh
         if not isinstance(m, StructuredMesh) or not lattice_fits(m.nx, m.ny):
             return None
-        gx, gy, kappa = lattice_means(m, eps)
-        if not kappa <= LATTICE_KAPPA:
+        gx, gy, self._kappa = lattice_means(m, eps)
+        # one right-hand side is where the diagonal form's iteration costs most
+        if not self._kappa <= LATTICE_KAPPA or not lattice_pays(m, self._kappa, 1):
             return None
         L = N.lib()
         nbytes = C.c_size_t()
@@ -136,7 +163,7 @@ class PoissonProblem:
         if self._plan is not None and max_iter >= 16 * (self.mesh.nx + self.mesh.ny) + 256:
             r = rho if isinstance(rho, torch.Tensor) else torch.from_numpy(np.asarray(rho, np.float64))
             r = r.to(self.device, torch.float64).reshape(n, -1).contiguous()
-            if r.shape[1] <= LATTICE_MAX_RHS:
+            if r.shape[1] <= LATTICE_MAX_RHS and lattice_pays(self.mesh, self._kappa, r.shape[1]):
                 return self._solve_lattice(r, V_p, V_n, tol, max_iter, x0)
             rho = r
         b = self.rhs(rho)

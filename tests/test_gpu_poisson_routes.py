@@ -41,9 +41,37 @@ def test_plan_is_bounded():
     assert L.qd_poisson_lattice_workspace_size(8, P.LATTICE_MAX_NY + 1, 1, C.byref(size)) != N.QD_OK
 
 
+# nx, ny, kappa, right-hand sides, whether the lattice form was the faster one,
+# timed with eps varying at random (kappa 1: along x only)
+TIMED = [(300, 100, 35.8, 64, True), (100, 50, 1.0, 1, True), (1000, 1000, 32.6, 16, True),
+         (4000, 16, 56.1, 64, True), (8, 4096, 1.0, 64, True), (32, 512, 8.4, 64, True),
+         (8, 512, 30.0, 64, False), (8, 2048, 29.4, 1, False), (8, 4096, 8.0, 64, False),
+         (2, 2048, 1.4, 64, False), (32, 2048, 30.4, 64, False), (4, 4, 22.5, 64, False)]
+
+
+@pytest.mark.parametrize("nx,ny,kappa,nrhs,lattice", TIMED)
+def test_rule_takes_the_form_that_was_faster(nx, ny, kappa, nrhs, lattice):
+    from qdsim_b200 import mesh as Mh, poisson as P
+    m = Mh.StructuredMesh(1, nx, ny, float(nx), float(ny))
+    assert P.lattice_pays(m, kappa, nrhs) == lattice
+
+
 @pytest.mark.gpu
 def test_a_tall_narrow_mesh_takes_the_diagonal_form(cuda):
     om, m = _mesh(4, 12000)
     eps = np.random.default_rng(1).uniform(10.0, 14.0, om.num_elements)
     prob, err = _solve(cuda, om, m, eps, 2)
     assert prob._plan is None and err <= 1e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nrhs,contrast,plan", [
+    (32, 1024, 64, 30.0, True),     # one right-hand side pays, 64 do not
+    (8, 1024, 1, 8.0, True),
+    (2, 2048, 3, 8.0, False),       # never pays: no plan
+])
+def test_narrow_meshes_match_the_oracle(cuda, nx, ny, nrhs, contrast, plan):
+    om, m = _mesh(nx, ny, hy=2.0)
+    eps = np.exp(np.random.default_rng(nx).uniform(0.0, np.log(contrast), om.num_elements))
+    prob, err = _solve(cuda, om, m, eps, nrhs)
+    assert (prob._plan is not None) == plan and err <= 1e-9
