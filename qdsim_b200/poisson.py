@@ -143,6 +143,15 @@ class PoissonProblem:
         torch.cuda.current_stream().synchronize()
         return plan
 
+    def _least_cap(self, tol):
+        """The iteration cap from which the lattice form is taken.  It must be
+        enough for that form, which needs at most sqrt(kappa) / 2 ln(2 / tol)
+        iterations and a few more for the residual's scale; and below nx / 2 the
+        call is left to end at its cap as the diagonal form does, whose iterations
+        carry a contact's value one column further each."""
+        digits = math.log(2.0 / min(tol, 1.0)) if tol > 0.0 else 0.0
+        return max(1.0, self.mesh.nx / 2, 0.5 * math.sqrt(self._kappa) * (digits + 8.0))
+
     def rhs(self, rho):
         """(1e-18/eps0) M (-rho) on the device; rho [N] or [N, nrhs] (C/m^3)."""
         r = rho if isinstance(rho, torch.Tensor) else torch.from_numpy(np.asarray(rho, np.float64))
@@ -157,10 +166,7 @@ class PoissonProblem:
     def solve(self, rho, V_p, V_n, tol=1e-12, max_iter=20000, x0=None):
         """phi (V) at every node, [N] or [N, nrhs] (device tensor)."""
         n = self.mesh.num_nodes
-        # The cap counts iterations of the diagonal form, which needs about
-        # 3 max(nx, ny): a call capped below any count that could converge is
-        # left with that form, so that it ends at its cap as it always did.
-        if self._plan is not None and max_iter >= 16 * (self.mesh.nx + self.mesh.ny) + 256:
+        if self._plan is not None and max_iter >= self._least_cap(tol):
             r = rho if isinstance(rho, torch.Tensor) else torch.from_numpy(np.asarray(rho, np.float64))
             r = r.to(self.device, torch.float64).reshape(n, -1).contiguous()
             if r.shape[1] <= LATTICE_MAX_RHS and lattice_pays(self.mesh, self._kappa, r.shape[1]):

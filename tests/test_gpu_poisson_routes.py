@@ -75,3 +75,30 @@ def test_narrow_meshes_match_the_oracle(cuda, nx, ny, nrhs, contrast, plan):
     eps = np.exp(np.random.default_rng(nx).uniform(0.0, np.log(contrast), om.num_elements))
     prob, err = _solve(cuda, om, m, eps, nrhs)
     assert (prob._plan is not None) == plan and err <= 1e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,kw", [
+    (1000, 300, {}),                        # large meshes at the default cap
+    (300, 100, {"max_iter": 5000}),         # caps that are enough for either form
+    (300, 100, {"max_iter": 1000}),
+    (60, 30, {"max_iter": 60}),
+])
+def test_the_cap_does_not_choose_the_form(cuda, nx, ny, kw):
+    """The lattice form's iterations do not grow with the mesh: at most 14 here (eps
+    in 10..14), where the diagonal form takes more than 3 per column."""
+    om, m = _mesh(nx, ny)
+    eps = np.random.default_rng(nx).uniform(10.0, 14.0, om.num_elements)
+    prob, err = _solve(cuda, om, m, eps, 1, **kw)
+    assert prob.last_iters <= 14 and err <= 1e-9
+
+
+@pytest.mark.gpu
+def test_a_cap_that_is_enough_for_the_diagonal_form_only(cuda):
+    """15 unknowns: the diagonal form ends within 15 iterations, the lattice form's
+    bound is 30 at this contrast."""
+    om, m = _mesh(4, 4)
+    eps = np.exp(np.random.default_rng(5).uniform(0.0, np.log(8.0), om.num_elements))
+    prob, err = _solve(cuda, om, m, eps, 1, max_iter=18)
+    assert prob._plan is not None and err <= 1e-9
+    assert prob._least_cap(1e-12) > 18
