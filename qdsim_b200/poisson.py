@@ -95,9 +95,11 @@ def lattice_means(mesh, eps):
     gx, gy = ex.sum(0) / ny, ey.sum(0) / ny
     w = np.ones(ny + 1)
     w[0] = w[-1] = 0.5
-    inner = ey[:, 1:-1] / gy[1:-1]           # the end columns are Dirichlet
-    q = np.concatenate([(ex / (w[:, None] * gx)).ravel(), inner.ravel()])
-    kappa = float(q.max() / q.min()) if q.min() > 0.0 and np.isfinite(q.max()) else np.inf
+    with np.errstate(divide="ignore", invalid="ignore"):
+        inner = ey[:, 1:-1] / gy[1:-1]       # the end columns are Dirichlet
+        q = np.concatenate([(ex / (w[:, None] * gx)).ravel(), inner.ravel()])
+    positive = gx.min() > 0.0 and gy.min() > 0.0 and q.min() > 0.0    # not with NaN
+    kappa = float(q.max() / q.min()) if positive and np.isfinite(q.max()) else np.inf
     return gx, gy, kappa
 
 

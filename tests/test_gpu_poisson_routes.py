@@ -41,6 +41,19 @@ def test_plan_is_bounded():
     assert L.qd_poisson_lattice_workspace_size(8, P.LATTICE_MAX_NY + 1, 1, C.byref(size)) != N.QD_OK
 
 
+@pytest.mark.filterwarnings("error")
+def test_no_plan_without_positive_conductances():
+    """The separable operator must be positive definite; zero, negative and non-finite
+    columns leave the problem to the diagonal form, without a warning."""
+    from qdsim_b200 import mesh as Mh, poisson as P
+    m = Mh.StructuredMesh(1, 6, 4, 6.0, 4.0)
+    for bad in (-3.0, 0.0, np.nan, np.inf):
+        assert P.lattice_means(m, np.full(m.num_elements, bad))[2] == np.inf
+        eps = np.full((4, 6, 2), 2.0)
+        eps[:, 2] = bad
+        assert P.lattice_means(m, eps.ravel())[2] == np.inf
+
+
 # nx, ny, kappa, right-hand sides, whether the lattice form was the faster one,
 # timed with eps varying at random (kappa 1: along x only)
 TIMED = [(300, 100, 35.8, 64, True), (100, 50, 1.0, 1, True), (1000, 1000, 32.6, 16, True),
