@@ -207,6 +207,9 @@ typedef struct {
   int32_t setup_cached;
 } qd_lobpcg_opts;
 
+/* Bytes of a workspace for a batch of n_dots dots, n_rows_total rows and nnz_total
+ * nonzeros.  It also serves every batch with no more of each (same b, prec_mode and
+ * options; without preconditioner, or with lattices no larger). */
 int qd_lobpcg_workspace_size(int32_t n_dots, int64_t n_rows_total, int64_t nnz_total, int b,
                              int prec_mode, const qd_dst_prec *h_prec,
                              const qd_lobpcg_opts *opts, size_t *bytes);

@@ -58,10 +58,14 @@ namespace {
 // solves at 1024 / 512 / 256 / 128 rows per chunk: 4.9k rows 9.9 / 9.7 / 9.4 /
 // 8.6 ms, 19k rows - / 17.1 / 16.9 / 13.9, 59k rows - / 27.1 / 28.8 / 32.8, 188k rows
 // 27.3 / 26.3 / 24.7 / 28.0, 473k rows 51.6 / 49.8 / 55.8 / 72.3.
+struct ChunkStep { int64_t rows; int chunk; };
+constexpr ChunkStep kChunkSteps[] = {{32768, 128}, {300000, 512}};   // up to these rows
 int chunk_rows_of(const qd_lobpcg_opts *opts, int64_t n_rows) {
   const int c = opts ? opts->chunk_rows : 0;
   if (c >= 256 && c <= 8192 && c % 64 == 0) return c;
-  return n_rows <= 32768 ? 128 : n_rows <= 300000 ? 512 : 1024;
+  for (const ChunkStep &t : kChunkSteps)
+    if (n_rows <= t.rows) return t.chunk;
+  return 1024;
 }
 constexpr int kMaxB = 16;
 constexpr int kMaxM = 3 * kMaxB;
@@ -3381,16 +3385,24 @@ extern "C" int qd_lobpcg_workspace_size(int32_t n_dots, int64_t n_rows_total,
   if (!bytes || n_dots <= 0 || n_rows_total <= 0 || nnz_total <= 0 || b < 4 || b > kMaxB ||
       b % 4)
     return QD_ERR_INVALID;
-  // upper bound on the chunk count: every dot contributes at most one partial chunk
-  const int chunk_rows = chunk_rows_of(opts, n_rows_total);
-  const int nchunks = int(n_rows_total / chunk_rows) + n_dots;
   int64_t ntx = 0, nty = 0;
   if (h_prec) qd::dst_tiles(n_dots, h_prec, b, nullptr, &ntx, nullptr, &nty);
-  qd::Arena ar(nullptr, 0);
-  Layout L;
-  carve(ar, n_dots, n_rows_total, nnz_total, b, nchunks, chunk_rows, ntx, nty,
-        prec_mode == QD_PREC_MIXED, needs_jacobi(n_dots, h_prec), L);
-  *bytes = ar.used;
+  auto need = [&](int64_t rows) {
+    // upper bound on the chunk count: every dot contributes at most one partial chunk
+    const int chunk_rows = chunk_rows_of(opts, rows);
+    const int nchunks = int(rows / chunk_rows) + n_dots;
+    qd::Arena ar(nullptr, 0);
+    Layout L;
+    carve(ar, n_dots, rows, nnz_total, b, nchunks, chunk_rows, ntx, nty,
+          prec_mode == QD_PREC_MIXED, needs_jacobi(n_dots, h_prec), L);
+    return ar.used;
+  };
+  size_t most = need(n_rows_total);
+  // fewer rows may mean shorter chunks and more partial sums: a workspace also
+  // serves every smaller batch
+  for (const ChunkStep &t : kChunkSteps)
+    if (t.rows < n_rows_total) most = std::max(most, need(t.rows));
+  *bytes = most;
   return QD_OK;
 }
 
