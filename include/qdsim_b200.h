@@ -186,7 +186,7 @@ typedef struct {
  *                (levels near zero energy); <= 0: purely relative
  *   chunk_rows   rows per chunk, the CTA unit of every row-parallel kernel
  *                (SpMM, Gram, orthogonalisation, update) and of the per-chunk
- *                partial sums; a multiple of 64 in [256, 8192], else
+ *                partial sums; a multiple of 64 in [128, 8192], else
  *                128 (batches up to 32,768 rows), 512 (up to 300,000) or 1024
  *   setup_cached nonzero: the caller asserts that d_work, d_rowptr and d_col
  *                (and their contents) are those of the previous call with

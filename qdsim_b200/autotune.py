@@ -34,7 +34,7 @@ DEFAULT_CACHE = Path(__file__).resolve().parent / "tuned.json"
 DEFAULTS = {"block": 12, "shift_ev": 0.02, "stag_window": 12, "tol32": 1e-7,
             "chunk_rows": 1024}
 SPACE = {
-    "chunk_rows": [512, 1024, 2048, 4096],
+    "chunk_rows": [128, 256, 512, 1024, 2048, 4096],
     "shift_ev": [0.01, 0.02, 0.04],
     "block": [12, 16],
     "stag_window": [8, 12, 20],

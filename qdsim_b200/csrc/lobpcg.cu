@@ -53,7 +53,7 @@
 namespace {
 
 // Rows per chunk (the CTA unit of every row-parallel kernel): the option's
-// value when it is a multiple of 64 in [256, 8192], else by the batch's rows, so
+// value when it is a multiple of 64 in [128, 8192], else by the batch's rows, so
 // that small batches have enough CTAs and large ones few partial sums.  Whole
 // solves at 1024 / 512 / 256 / 128 rows per chunk: 4.9k rows 9.9 / 9.7 / 9.4 /
 // 8.6 ms, 19k rows - / 17.1 / 16.9 / 13.9, 59k rows - / 27.1 / 28.8 / 32.8, 188k rows
@@ -62,7 +62,7 @@ struct ChunkStep { int64_t rows; int chunk; };
 constexpr ChunkStep kChunkSteps[] = {{32768, 128}, {300000, 512}};   // up to these rows
 int chunk_rows_of(const qd_lobpcg_opts *opts, int64_t n_rows) {
   const int c = opts ? opts->chunk_rows : 0;
-  if (c >= 256 && c <= 8192 && c % 64 == 0) return c;
+  if (c >= 128 && c <= 8192 && c % 64 == 0) return c;
   for (const ChunkStep &t : kChunkSteps)
     if (n_rows <= t.rows) return t.chunk;
   return 1024;

@@ -150,7 +150,7 @@ def lobpcg_packed(row_off, rowptr, col, H, M, k, b=None, precision="mixed", tol=
     warm-starts the first k block vectors; ``eig_scale`` (eV) measures
     eigenvalue errors relative to max(|E|, eig_scale) (levels near zero);
     ``chunk_rows`` sets the rows per CTA of the row-parallel kernels (a
-    multiple of 64 in [256, 8192]; ``None``: by the batch's size); ``setup_cached`` asserts
+    multiple of 64 in [128, 8192]; ``None``: by the batch's size); ``setup_cached`` asserts
     that the workspace and the CSR pattern are those of the previous call with
     this workspace (repeated solves of one batch: no read-back and no copy of
     unchanged tables during the set-up)."""
