@@ -1761,7 +1761,12 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
       double *s_piv = sE;      // [m]
       chol = chol_congruence<TM>(Bt, T, N, mu, 2 * B, pivot_floor, sW, s_piv);
       if (chol) {
-        // the diagonal factor; Q[i][c] = N[c][i] / sqrt(piv_c)
+        // the diagonal factor; Q[i][c] = N[c][i] / sqrt(piv_c).  The elimination
+        // rounds (i, j) and (j, i) differently and the factor magnifies that, to
+        // 1e-12 of |T|: the half sum is what is accurate (to 1e-16 in the levels;
+        // the tridiagonalisation of T as it stands gave 1e-14, up to 1e-12)
+        static_assert(S + 1 <= 2 * m, "T fits in A' and B'");
+        double *sTt = sA;
         if (tid < S) s_red[tid] = tid < mu && s_piv[tid] > 0.0 ? rsqrt(s_piv[tid]) : 0.0;
         __syncthreads();
         double fro = 0.0;
@@ -1773,7 +1778,10 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
             const double si = s_red[i];
             T.v[a][b] = si != 0.0 && s_red[j] != 0.0 ? T.v[a][b] * (si * s_red[j]) : 0.0;
             fro = fma(T.v[a][b], T.v[a][b], fro);
-            if (i < m && j < m) sT[j * m + i] = si != 0.0 ? N.v[a][b] * si : 0.0;
+            if (i < m && j < m) {
+              sT[j * m + i] = si != 0.0 ? N.v[a][b] * si : 0.0;
+              sTt[i * (S + 1) + j] = T.v[a][b];
+            }
           }
 #pragma unroll
         for (int o = 16; o; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
@@ -1785,6 +1793,11 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
 #pragma unroll
         for (int a = 0; a < TM; ++a) {
           const int i = ty + 16 * a;
+#pragma unroll
+          for (int b = 0; b < TM; ++b) {
+            const int j = tx + 16 * b;
+            if (i < m && j < m) T.v[a][b] = 0.5 * (T.v[a][b] + sTt[j * (S + 1) + i]);
+          }
           if (tx == ty && i < m && s_red[i] == 0.0) T.v[a][a] = above;
         }
         __syncthreads();
