@@ -35,15 +35,15 @@ std::atomic<uint64_t> g_launches{0};
 
 namespace {
 
-// Rows per block, threads per block and element-matrix entries staged at once,
-// by nodes per element.  A structured P1 / P2 / P3 mesh has at most 18 / 24 / 33
+// Most and least rows per block, threads per block and element-matrix entries staged
+// at once, by nodes per element.  A structured P1 / P2 / P3 mesh has at most 18 / 24 / 33
 // entries per row on average over a lattice line, so one pass of a block takes
 // all of its rows; rows of higher valence (refined meshes, up to 16 elements)
 // take more passes.
 template <int K> struct AsmShape;
-template <> struct AsmShape<3> { static constexpr int ROWS = 128, THREADS = 256, CAP = 2304; };
-template <> struct AsmShape<6> { static constexpr int ROWS = 96, THREADS = 256, CAP = 2304; };
-template <> struct AsmShape<10> { static constexpr int ROWS = 64, THREADS = 128, CAP = 2240; };
+template <> struct AsmShape<3> { static constexpr int ROWS = 128, LEAST = 16, THREADS = 256, CAP = 2304; };
+template <> struct AsmShape<6> { static constexpr int ROWS = 96, LEAST = 16, THREADS = 256, CAP = 2304; };
+template <> struct AsmShape<10> { static constexpr int ROWS = 64, LEAST = 8, THREADS = 128, CAP = 2240; };
 
 // Shared memory of a block, bytes.  Tables: M, Sxx, Sxy, Syy as [a][b] and the
 // potential weights as [a][b][l], rows padded so that lanes with different a
@@ -110,14 +110,14 @@ __device__ __forceinline__ void stage_bytes(uint8_t *dst, const uint8_t *src, in
 // reference-compatible P1 modes.
 template <int K, bool HAS_W, bool FEM>
 __global__ void __launch_bounds__(AsmShape<K>::THREADS)
-assemble_rows_kernel(int mode, int32_t n, int pairs8, const double2 *__restrict__ nodes,
+assemble_rows_kernel(int mode, int32_t n, int rows, int pairs8, const double2 *__restrict__ nodes,
                      const int32_t *__restrict__ elems, const double *__restrict__ cvec,
                      const double *__restrict__ V, const double *__restrict__ W,
                      const int32_t *__restrict__ rowptr, const int32_t *__restrict__ adjptr,
                      const int32_t *__restrict__ adj, const int32_t *__restrict__ cptr,
                      const uint8_t *__restrict__ contrib, const uint8_t *__restrict__ slotcnt,
                      double *__restrict__ H, double *__restrict__ M, double *__restrict__ Him,
-                     int32_t *__restrict__ status) {
+                     int32_t *__restrict__ status, const double *__restrict__ tables) {
   using LY = AsmLayout<K, HAS_W>;
   constexpr int ROWS = AsmShape<K>::ROWS, TH = AsmShape<K>::THREADS, CAP = LY::CAP, KP = LY::KP;
   constexpr int KK = K * K, B0 = TabBase<K>::v;
@@ -133,15 +133,15 @@ assemble_rows_kernel(int mode, int32_t n, int pairs8, const double2 *__restrict_
   const int tid = threadIdx.x;
   for (int i = tid; i < 4 * KK + K * KK; i += TH) {
     if (i < 4 * KK) {
-      s_tab[i] = c_tab[B0 + i];
+      s_tab[i] = tables[B0 + i];
     } else {
       const int l = (i - 4 * KK) / KK, ab = (i - 4 * KK) % KK;
-      s_tab[LY::NT + ab / K * LY::TP + ab % K * K + l] = c_tab[B0 + i];
+      s_tab[LY::NT + ab / K * LY::TP + ab % K * K + l] = tables[B0 + i];
     }
   }
-  const int64_t step = int64_t(gridDim.x) * ROWS;
-  for (int64_t r0 = int64_t(blockIdx.x) * ROWS; r0 < n; r0 += step) {
-    const int nrows = int(min(int64_t(ROWS), n - r0));
+  const int64_t step = int64_t(gridDim.x) * rows;
+  for (int64_t r0 = int64_t(blockIdx.x) * rows; r0 < n; r0 += step) {
+    const int nrows = int(min(int64_t(rows), n - r0));
     for (int i = tid; i <= nrows; i += TH) {
       s_adj[i] = adjptr[r0 + i];
       s_rp[i] = rowptr[r0 + i];
@@ -168,9 +168,12 @@ assemble_rows_kernel(int mode, int32_t n, int pairs8, const double2 *__restrict_
       const uint8_t *con = asm_sm + LY::con + (reinterpret_cast<uintptr_t>(contrib + c0) & 3);
       const uint8_t *sc = asm_sm + LY::cnt + (reinterpret_cast<uintptr_t>(slotcnt + rp0) & 3);
       if (tid == 0) s_nheavy = 0;
-      // (1); a thread reads back the pairs that it copied itself
+      // (1); P3 and few pairs: `parts` threads share a pair's entries
+      const int parts = K < 10 || 2 * na > TH ? 1 : (5 * na > TH ? 2 : 5);
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      for (int p = tid; p < na; p += TH) {
+      if (parts > 1) __syncthreads();   // else a thread reads the pairs that it copied itself
+      for (int item = tid; item < na * parts; item += TH) {
+        const int p = K < 10 ? item : item / parts, part = K < 10 ? 0 : item - p * parts;
         const int packed = s_pair[p], e = packed >> 4, a = packed & 15;
         int g[K];
         const int32_t *ep = elems + size_t(e) * K;
@@ -212,7 +215,7 @@ assemble_rows_kernel(int mode, int32_t n, int pairs8, const double2 *__restrict_
         if (!(det != 0.0) || !isfinite(det) || !isfinite(ce)) atomicOr(status, 1);
         const double *Mr = s_tab + a * K, *T = s_tab + LY::NT + a * LY::TP;
 #pragma unroll(K <= 6 ? K : 2)
-        for (int b = 0; b < K; ++b) {
+        for (int b = part; b < K; b += parts) {
           const double st = g00 * Mr[KK + b] + g01 * Mr[2 * KK + b] + g11 * Mr[3 * KK + b];
           double hk, mk = A * Mr[b];
           if constexpr (FEM) {
@@ -338,11 +341,15 @@ int launch_rows(int mode, int32_t n, const double *nodes, const int32_t *elems, 
                 const double *V, const double *W, const int32_t *rowptr, const int32_t *adjptr,
                 const int32_t *adj, const int32_t *cptr, const uint8_t *contrib,
                 const uint8_t *slotcnt, double *H, double *M, double *Him, int32_t *status,
-                cudaStream_t s) {
+                const double *tables, cudaStream_t s) {
   constexpr size_t smem = AsmLayout<K, HAS_W>::bytes;
   QD_CUDA_TRY(cudaFuncSetAttribute(assemble_rows_kernel<K, HAS_W, FEM>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  // a block builds its tables once: as many blocks as are resident
+  // a block builds its tables once: as many blocks as are resident, and on small
+  // meshes no more rows per block than it takes to give each of them some (at the
+  // most rows per block P1 100 x 50 cells took 8.5 us and P3 16 x 8 cells 16.4, the row
+  // per 8 to 32 lanes before 6.8 and 11.3; with fewer rows, and for P3 threads that
+  // share a pair, 6.2 and 10.2)
   static std::atomic<int> per_sm{0};
   int res = per_sm.load(std::memory_order_relaxed);
   if (res == 0) {
@@ -351,12 +358,15 @@ int launch_rows(int mode, int32_t n, const double *nodes, const int32_t *elems, 
     if (res < 1) return QD_ERR_CUDA;
     per_sm.store(res, std::memory_order_relaxed);
   }
-  const int64_t chunks = (int64_t(n) + AsmShape<K>::ROWS - 1) / AsmShape<K>::ROWS;
-  const int blocks = int(std::min<int64_t>(chunks, int64_t(res) * 148));
+  const int64_t resident = int64_t(res) * 148;
+  const int rows = int(std::clamp<int64_t>((n + resident - 1) / resident, AsmShape<K>::LEAST,
+                                           AsmShape<K>::ROWS));
+  const int64_t chunks = (int64_t(n) + rows - 1) / rows;
+  const int blocks = int(std::min<int64_t>(chunks, resident));
   qd::prof_begin(qd::PK_ASSEMBLE, s);
   assemble_rows_kernel<K, HAS_W, FEM><<<blocks, AsmShape<K>::THREADS, smem, s>>>(
-      mode, n, reinterpret_cast<uintptr_t>(elems) % 8 == 0, reinterpret_cast<const double2 *>(nodes),
-      elems, c, V, W, rowptr, adjptr, adj, cptr, contrib, slotcnt, H, M, Him, status);
+      mode, n, rows, reinterpret_cast<uintptr_t>(elems) % 8 == 0, reinterpret_cast<const double2 *>(nodes),
+      elems, c, V, W, rowptr, adjptr, adj, cptr, contrib, slotcnt, H, M, Him, status, tables);
   qd::prof_end(qd::PK_ASSEMBLE, s);
   QD_CHECK_LAUNCH();
   return QD_OK;
@@ -367,18 +377,18 @@ int launch_assemble(int mode, int32_t n, const double *nodes, const int32_t *ele
                     const double *c, const double *V, const double *W, const int32_t *rowptr,
                     const int32_t *adjptr, const int32_t *adj, const int32_t *cptr,
                     const uint8_t *contrib, const uint8_t *slotcnt, double *H, double *M,
-                    double *Him, int32_t *status, cudaStream_t s) {
+                    double *Him, int32_t *status, const double *tables, cudaStream_t s) {
   if (n == 0) return QD_OK;
   if constexpr (K == 3) {   // the reference-compatible modes are P1
     if (mode != QD_ASM_FEM)
       return launch_rows<K, false, false>(mode, n, nodes, elems, c, V, W, rowptr, adjptr, adj, cptr,
-                                          contrib, slotcnt, H, M, Him, status, s);
+                                          contrib, slotcnt, H, M, Him, status, tables, s);
   }
   if (W)
     return launch_rows<K, true, true>(mode, n, nodes, elems, c, V, W, rowptr, adjptr, adj, cptr,
-                                      contrib, slotcnt, H, M, Him, status, s);
+                                      contrib, slotcnt, H, M, Him, status, tables, s);
   return launch_rows<K, false, true>(mode, n, nodes, elems, c, V, W, rowptr, adjptr, adj, cptr,
-                                     contrib, slotcnt, H, M, Him, status, s);
+                                     contrib, slotcnt, H, M, Him, status, tables, s);
 }
 
 }  // namespace
@@ -400,22 +410,23 @@ extern "C" int qd_assemble(int order, int mode, int64_t num_nodes, int64_t num_e
       !d_contrib || !d_slotcnt || !d_H || !d_M || !d_status)
     return QD_ERR_INVALID;
   if (reinterpret_cast<uintptr_t>(d_nodes) % 16 != 0) return QD_ERR_INVALID;
-  int st = ensure_tables();
+  const double *tables = nullptr;
+  int st = ensure_tables(&tables);
   if (st != QD_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (order) {
     case 1:
       return launch_assemble<3>(mode, n_dofs, d_nodes, d_elems, d_c, d_V, d_W, d_rowptr,
                                 d_adjptr, d_adj, d_cptr, d_contrib, d_slotcnt, d_H, d_M,
-                                d_Himag, d_status, s);
+                                d_Himag, d_status, tables, s);
     case 2:
       return launch_assemble<6>(mode, n_dofs, d_nodes, d_elems, d_c, d_V, d_W, d_rowptr,
                                 d_adjptr, d_adj, d_cptr, d_contrib, d_slotcnt, d_H, d_M,
-                                d_Himag, d_status, s);
+                                d_Himag, d_status, tables, s);
     default:
       return launch_assemble<10>(mode, n_dofs, d_nodes, d_elems, d_c, d_V, d_W, d_rowptr,
                                  d_adjptr, d_adj, d_cptr, d_contrib, d_slotcnt, d_H, d_M,
-                                 d_Himag, d_status, s);
+                                 d_Himag, d_status, tables, s);
   }
 }
 

@@ -21,18 +21,29 @@ template <> struct TabBase<10> { static constexpr int v = 423; };
 
 std::mutex g_tab_mu;
 bool g_tab_ready[64] = {false};
+const double *g_tab_addr[64] = {nullptr};
 
-int ensure_tables() {
+// Uploads the tables on first use; `addr` receives their address for kernels that
+// read them as global memory (copies to shared memory: lanes of a warp that read
+// different constants are served one by one).
+int ensure_tables(const double **addr = nullptr) {
   int dev = 0;
   QD_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return QD_ERR_LIMIT;
   std::lock_guard<std::mutex> lk(g_tab_mu);
-  if (g_tab_ready[dev]) return QD_OK;
+  if (g_tab_ready[dev]) {
+    if (addr) *addr = g_tab_addr[dev];
+    return QD_OK;
+  }
   static double host[qd::kTableDoubles];
   qd::TableOffsets off[4];
   qd::pack_tables(host, off);
   QD_CUDA_TRY(cudaMemcpyToSymbol(c_tab, host, sizeof(host)));
+  void *at = nullptr;
+  QD_CUDA_TRY(cudaGetSymbolAddress(&at, c_tab));
+  g_tab_addr[dev] = static_cast<const double *>(at);
   g_tab_ready[dev] = true;
+  if (addr) *addr = g_tab_addr[dev];
   return QD_OK;
 }
 
