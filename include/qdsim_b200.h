@@ -385,6 +385,13 @@ int qd_cap_spmm_lattice(int32_t n, int32_t width, int b, int vec_fp32, const int
                         const void *d_M, const void *d_X, int ldx, void *d_AX, void *d_MX, int ldy,
                         void *stream);
 
+/* qd_cap_spmm_lattice for a pattern of nnz nonzeros, by whose number per row (with
+ * b and n) the kernel is chosen; 0: not known.  The results are the same. */
+int qd_cap_spmm_pattern(int32_t n, int64_t nnz, int32_t width, int b, int vec_fp32,
+                        const int32_t *d_rowptr, const int32_t *d_col, const void *d_H,
+                        const void *d_Himag, const void *d_M, const void *d_X, int ldx, void *d_AX,
+                        void *d_MX, int ldy, void *stream);
+
 /* ---------------------------------------------------------------------------
  * Open-system eigensolve: the k eigenvalues nearest sigma of the complex-
  * symmetric pencil (H + i Himag, M), from block LOBPCG over the nev

@@ -68,6 +68,8 @@ SIGNATURES = {
     "qd_cap_spmm": (_int, [_i32, _int, _int, _p, _p, _p, _p, _p, _p, _int, _p, _p, _int, _p]),
     "qd_cap_spmm_lattice": (_int, [_i32, _i32, _int, _int, _p, _p, _p, _p, _p, _p, _int, _p, _p,
                                    _int, _p]),
+    "qd_cap_spmm_pattern": (_int, [_i32, _i64, _i32, _int, _int, _p, _p, _p, _p, _p, _p, _int, _p, _p,
+                                   _int, _p]),
     "qd_fe_interpolate": (_int, [_int, _i32, _i32, _dbl, _dbl, _int, _i64, _p, _i64, _p, _p,
                                  _p, _p, _p, _p, _int, _p]),
     "qd_bounded_wait_selftest": (_int, [_i64, _p, _int, _p, _p, _p]),

@@ -94,10 +94,10 @@ class CAPProblem:
             if T.stride(1) != 1 or T.shape[0] != self.n:
                 raise ValueError("cap spmm operands must be [n, b] with unit column stride")
         H, G, M = (self.H32, self.G32, self.M32) if fp32 else (self.H, self.G, self.M)
-        N.check(N.lib().qd_cap_spmm_lattice(
-            self.n, self._width, b, 1 if fp32 else 0, N.ptr(self.fem.d_rowptr), N.ptr(self.fem.d_col),
-            N.ptr(H), N.ptr(G), N.ptr(M), N.ptr(X), X.stride(0), N.ptr(AX), N.ptr(MX),
-            AX.stride(0), stream_ptr()), "qd_cap_spmm_lattice")
+        N.check(N.lib().qd_cap_spmm_pattern(
+            self.n, self.fem.nnz, self._width, b, 1 if fp32 else 0, N.ptr(self.fem.d_rowptr),
+            N.ptr(self.fem.d_col), N.ptr(H), N.ptr(G), N.ptr(M), N.ptr(X), X.stride(0), N.ptr(AX),
+            N.ptr(MX), AX.stride(0), stream_ptr()), "qd_cap_spmm_pattern")
 
     def precondition(self, R):
         """W = T R (real and imaginary parts as separate columns)."""

@@ -44,7 +44,7 @@ struct RowWalk {
   int i0, j0, place, left, run;
   __device__ RowWalk(const RowOrder &o, int half) {
     run = blockIdx.x;
-        place = half;
+    place = half;
     start(o);
   }
   __device__ void start(const RowOrder &o) {   // the first tile of run `run`
@@ -79,11 +79,82 @@ __device__ __forceinline__ int tiles_of(const RowOrder &o) {
   return sum;
 }
 
-// kLanes lanes per row; lane l owns columns l, l + 16, ... (C of them, so a
-// 48-column block keeps every lane busy), so each half-warp's vector loads are
-// 16 consecutive complex values.  The row's CSR entries are copied to shared
-// memory and read from there by all lanes (two or three reads per entry; by
-// shuffles it took seven).  A warp's two rows lie two apart: on a P2
+// Two kernels, the same sums in the same order (equal bits).  Both take kLanes
+// lanes per row; lane l owns columns l, l + 16, ... (C of them, so a 48-column
+// block keeps every lane busy), so each half-warp's vector loads are 16
+// consecutive complex values.
+//
+// cap_spmm_rows_kernel: a block per 16 rows; the row's CSR entries are loaded 16
+// at a time, one per lane, and broadcast by shuffles.  Small registers and no
+// set-up: where the vectors come from L2 and many rows in flight hide its latency
+// it is the faster one (tiles_pay).
+template <typename T, int C>
+__global__ void __launch_bounds__(kRowsPerBlock * kLanes, 4)
+cap_spmm_rows_kernel(int32_t n, int b, int ldx, int ldy, const int32_t *__restrict__ rowptr,
+                     const int32_t *__restrict__ col, const T *__restrict__ H,
+                     const T *__restrict__ G, const T *__restrict__ M,
+                     const typename Vec2<T>::type *__restrict__ X, typename Vec2<T>::type *AX,
+                     typename Vec2<T>::type *MX) {
+  using V = typename Vec2<T>::type;
+  const int row = blockIdx.x * kRowsPerBlock + (threadIdx.x / kLanes);
+  const int lane = threadIdx.x % kLanes;
+  // the two rows of a warp are independent: shuffles stay inside each half
+  const unsigned mask = 0xffffu << (threadIdx.x & 16);
+  const bool live = row < n;
+  T ar[C], ai[C], mr[C], mi[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) ar[c] = ai[c] = mr[c] = mi[c] = T(0);
+  const int p0 = live ? rowptr[row] : 0, p1 = live ? rowptr[row + 1] : 0;
+  for (int base = p0; base < p1; base += kLanes) {
+    const int p = base + lane;
+    int cj = 0;
+    T h = T(0), g = T(0), m = T(0);
+    if (p < p1) {
+      cj = col[p];
+      h = H[p];
+      g = G ? G[p] : T(0);
+      m = M[p];
+    }
+    const int cnt = min(kLanes, p1 - base);
+    for (int q = 0; q < cnt; ++q) {
+      const int j = __shfl_sync(mask, cj, q, kLanes);
+      const T hq = __shfl_sync(mask, h, q, kLanes);
+      const T gq = __shfl_sync(mask, g, q, kLanes);
+      const T mq = __shfl_sync(mask, m, q, kLanes);
+      const V *xr = X + size_t(j) * ldx;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int cc = c * kLanes + lane;
+        if (cc < b) {
+          const V x = xr[cc];
+          // (h + i g)(xr + i xi) = (h xr - g xi) + i (h xi + g xr)
+          ar[c] = fma(hq, x.x, fma(-gq, x.y, ar[c]));
+          ai[c] = fma(hq, x.y, fma(gq, x.x, ai[c]));
+          mr[c] = fma(mq, x.x, mr[c]);
+          mi[c] = fma(mq, x.y, mi[c]);
+        }
+      }
+    }
+  }
+  if (!live) return;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int cc = c * kLanes + lane;
+    if (cc < b) {
+      V a, mm;
+      a.x = ar[c];
+      a.y = ai[c];
+      mm.x = mr[c];
+      mm.y = mi[c];
+      AX[size_t(row) * ldy + cc] = a;
+      MX[size_t(row) * ldy + cc] = mm;
+    }
+  }
+}
+
+// cap_spmm_kernel: rows in tiles of the lattice (RowOrder).  The row's CSR entries
+// are copied to shared memory and read from there by all lanes (two or three reads
+// per entry; by shuffles it takes seven).  A warp's two rows lie two apart: on a P2
 // lattice neighbours have 19 and 9 entries, and half of the warp would wait.
 //
 // The latency of the gathers bounds it: a row reads 11 vector rows of 768 bytes
@@ -93,10 +164,16 @@ __device__ __forceinline__ int tiles_of(const RowOrder &o) {
 // one after it are on their way, and so are the vector rows of the next three
 // entries, also across the end of a row.  The warps of a block trade places from
 // tile to tile, so that none keeps the long rows.  FP64, b = 48, P2 400 x 200
-// cells: 378 us with a block per 16 rows of a line, shuffles and one entry's
-// loads in flight; now 257 us (FP32: 207 and 176 us).
+// cells: 376 us by cap_spmm_rows_kernel, 253 us here (FP32: 203 and 174 us).
 constexpr int kEntries = 24;        // entries staged at once (P1, P2: a whole row)
-constexpr int kAhead = 4;           // vector rows in flight per half-warp
+// Blocks per SM and vector rows in flight per half-warp.  FP64: with one column
+// per lane a fourth block fits; with four columns two rows in flight do without
+// spills (four of them spilled: P2 400 x 200, b = 49, 425 us, now 336).
+template <typename T, int C> struct TileShape { static constexpr int BLOCKS = 3, AHEAD = 4; };
+template <> struct TileShape<double, 1> { static constexpr int BLOCKS = 4, AHEAD = 4; };
+template <> struct TileShape<double, 2> { static constexpr int BLOCKS = 2, AHEAD = 4; };
+template <> struct TileShape<double, 3> { static constexpr int BLOCKS = 2, AHEAD = 4; };
+template <> struct TileShape<double, 4> { static constexpr int BLOCKS = 2, AHEAD = 2; };
 template <typename T> struct __align__(16) CsrEntry { T h, g, m; int j; };
 
 template <int N> __device__ __forceinline__ void copy_async(void *smem, const void *gmem) {
@@ -105,8 +182,7 @@ template <int N> __device__ __forceinline__ void copy_async(void *smem, const vo
 }
 
 template <typename T, int C>
-__global__ void __launch_bounds__(kRowsPerBlock * kLanes,
-                                  sizeof(T) == 4 || C < 2 ? 3 : 2)
+__global__ void __launch_bounds__(kRowsPerBlock * kLanes, TileShape<T, C>::BLOCKS)
 cap_spmm_kernel(RowOrder o, int b, int ldx, int ldy, const int32_t *__restrict__ rowptr,
                 const int32_t *__restrict__ col, const T *__restrict__ H,
                 const T *__restrict__ G, const T *__restrict__ M,
@@ -114,6 +190,7 @@ cap_spmm_kernel(RowOrder o, int b, int ldx, int ldy, const int32_t *__restrict__
                 typename Vec2<T>::type *MX) {
   using V = typename Vec2<T>::type;
   using Entry = CsrEntry<T>;
+  constexpr int kAhead = TileShape<T, C>::AHEAD;
   __shared__ Entry s_e[2][kRowsPerBlock][kEntries];
   const int lane = threadIdx.x % kLanes, half = threadIdx.x / kLanes;
   // the two rows of a warp are independent: barriers stay inside each half
@@ -236,35 +313,66 @@ cap_spmm_kernel(RowOrder o, int b, int ldx, int ldy, const int32_t *__restrict__
   }
 }
 
+// Whether the tiles are the faster form: by the type, the columns per lane, the
+// rows and the nonzeros per row z (P1 7, P2 11, P3 17), timed on lattices of 361 to
+// 319,000 rows with 1 to 64 columns against the rows kernel.  Gains and losses of
+// the tiles where they are taken, and why not elsewhere:
+//   FP64, 33 to 48 columns: 1.1 to 1.7 times faster everywhere; 49 to 64 columns:
+//     1.0 to 1.5; up to 16 columns: 1.0 to 1.5 from some thousand rows on.
+//   FP64, 17 to 32 columns: 1.04 to 1.12 on P2; P1 0.89 to 0.98, P3 0.90 to 0.98.
+//   FP32: 1.05 to 1.19 where X passes 19 MB (the traffic that tiles save is then
+//     what counts) and 1.0 to 1.06 on small P2 lattices up to 16 columns; 0.8 to
+//     1.0 otherwise and on P3; 49 to 64 columns 0.7 to 1.0.
+// z is not known (0) where the caller gives no pattern size: P2 is assumed.
+// Without a lattice the tiles are 16 rows of one line, and only the widest FP64
+// blocks gain (1.2 to 1.4 at 33 to 48 columns, P3 1.0).
+bool tiles_pay(bool fp32, int32_t n, int b, double z, bool lattice) {
+  if (z <= 0.0) z = 11.4;
+  const int c = (b + kLanes - 1) / kLanes;
+  if (fp32)
+    return lattice && c <= 3 && z < 14.0 &&
+           (int64_t(n) * b >= 2400000 || (c == 1 && z > 9.0 && n <= 32768));
+  if (!lattice) return c == 3;
+  return c == 1 ? n >= 2048 : c != 2 || (z > 9.0 && z < 14.0);
+}
+
 template <typename T, int C>
-int launch_c(RowOrder o, int b, int ldx, int ldy, const int32_t *rowptr, const int32_t *col,
-             const T *h, const T *g, const T *m, const typename Vec2<T>::type *x,
+int launch_c(RowOrder o, int32_t n, bool tiles, int b, int ldx, int ldy, const int32_t *rowptr,
+             const int32_t *col, const T *h, const T *g, const T *m, const typename Vec2<T>::type *x,
              typename Vec2<T>::type *ax, typename Vec2<T>::type *mx, cudaStream_t s) {
   constexpr int threads = kRowsPerBlock * kLanes;
-  static std::atomic<int> per_sm{0};
-  int res = per_sm.load(std::memory_order_relaxed);
-  if (res == 0) {
-    QD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, cap_spmm_kernel<T, C>, threads, 0));
-    if (res < 1) return QD_ERR_CUDA;
-    per_sm.store(res, std::memory_order_relaxed);
+  if constexpr (sizeof(T) == 8 || C <= 3) {
+    if (tiles) {
+      static std::atomic<int> per_sm{0};
+      int res = per_sm.load(std::memory_order_relaxed);
+      if (res == 0) {
+        QD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, cap_spmm_kernel<T, C>, threads, 0));
+        if (res < 1) return QD_ERR_CUDA;
+        per_sm.store(res, std::memory_order_relaxed);
+      }
+      // runs of 8 tiles (longer ones share no more, and leave the last wave
+      // emptier: 276 us at 25), shorter where a block would have fewer than four
+      const int bands = (o.lines - 1) / (16 >> o.shift) + 1;
+      const int64_t count = int64_t(o.tiles_i) * bands, resident = int64_t(res) * 148;
+      o.run = int(std::max<int64_t>(1, std::min<int64_t>(8, count / (4 * resident))));
+      o.runs_i = (o.tiles_i - 1) / o.run + 1;
+      o.runs = o.runs_i * bands;
+      const unsigned blocks = unsigned(std::min<int64_t>(o.runs, resident));
+      cap_spmm_kernel<T, C><<<blocks, threads, 0, s>>>(o, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx);
+      QD_CHECK_LAUNCH();
+      return QD_OK;
+    }
   }
-  // runs of 8 tiles (longer ones share no more, and leave the last wave
-  // emptier: 276 us at 25), shorter where a block would have fewer than four
-  const int bands = (o.lines - 1) / (16 >> o.shift) + 1;
-  const int64_t tiles = int64_t(o.tiles_i) * bands, resident = int64_t(res) * 148;
-  o.run = int(std::max<int64_t>(1, std::min<int64_t>(8, tiles / (4 * resident))));
-  o.runs_i = (o.tiles_i - 1) / o.run + 1;
-  o.runs = o.runs_i * bands;
-  const unsigned blocks = unsigned(std::min<int64_t>(o.runs, resident));
-  cap_spmm_kernel<T, C><<<blocks, threads, 0, s>>>(o, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx);
+  const unsigned blocks = unsigned((int64_t(n) + kRowsPerBlock - 1) / kRowsPerBlock);
+  cap_spmm_rows_kernel<T, C><<<blocks, threads, 0, s>>>(n, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx);
   QD_CHECK_LAUNCH();
   return QD_OK;
 }
 
 template <typename T>
-int launch(int32_t n, int width, int b, int ldx, int ldy, const int32_t *rowptr,
-           const int32_t *col, const void *H, const void *G, const void *M, const void *X, void *AX, void *MX,
-           cudaStream_t s) {
+int launch(int32_t n, int64_t nnz, int width, int b, int ldx, int ldy, const int32_t *rowptr,
+           const int32_t *col, const void *H, const void *G, const void *M, const void *X, void *AX,
+           void *MX, cudaStream_t s) {
   using V = typename Vec2<T>::type;
   const T *h = static_cast<const T *>(H), *g = static_cast<const T *>(G),
           *m = static_cast<const T *>(M);
@@ -277,37 +385,47 @@ int launch(int32_t n, int width, int b, int ldx, int ldy, const int32_t *rowptr,
   o.lines = n / o.width;
   o.shift = lattice ? 2 : 4;
   o.tiles_i = ((o.width - 1) >> o.shift) + 1;
+  const bool t = tiles_pay(sizeof(T) == 4, n, b, double(nnz) / n, lattice);
   switch ((b + kLanes - 1) / kLanes) {
-    case 1: return launch_c<T, 1>(o, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
-    case 2: return launch_c<T, 2>(o, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
-    case 3: return launch_c<T, 3>(o, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
-    default: return launch_c<T, 4>(o, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
+    case 1: return launch_c<T, 1>(o, n, t, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
+    case 2: return launch_c<T, 2>(o, n, t, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
+    case 3: return launch_c<T, 3>(o, n, t, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
+    default: return launch_c<T, 4>(o, n, t, b, ldx, ldy, rowptr, col, h, g, m, x, ax, mx, s);
   }
 }
 
 }  // namespace
+
+extern "C" int qd_cap_spmm_pattern(int32_t n, int64_t nnz, int32_t width, int b, int vec_fp32,
+                                   const int32_t *d_rowptr, const int32_t *d_col,
+                                   const void *d_H, const void *d_Himag, const void *d_M,
+                                   const void *d_X, int ldx, void *d_AX, void *d_MX, int ldy,
+                                   void *stream) {
+  if (n < 0 || nnz < 0 || b < 1 || b > 64 || ldx < b || ldy < b || !d_rowptr || !d_col || !d_H ||
+      !d_M || !d_X || !d_AX || !d_MX)
+    return QD_ERR_INVALID;
+  if (n == 0) return QD_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (vec_fp32)
+    return launch<float>(n, nnz, width, b, ldx, ldy, d_rowptr, d_col, d_H, d_Himag, d_M, d_X, d_AX,
+                         d_MX, s);
+  return launch<double>(n, nnz, width, b, ldx, ldy, d_rowptr, d_col, d_H, d_Himag, d_M, d_X, d_AX,
+                        d_MX, s);
+}
 
 extern "C" int qd_cap_spmm_lattice(int32_t n, int32_t width, int b, int vec_fp32,
                                    const int32_t *d_rowptr, const int32_t *d_col,
                                    const void *d_H, const void *d_Himag, const void *d_M,
                                    const void *d_X, int ldx, void *d_AX, void *d_MX, int ldy,
                                    void *stream) {
-  if (n < 0 || b < 1 || b > 64 || ldx < b || ldy < b || !d_rowptr || !d_col || !d_H || !d_M ||
-      !d_X || !d_AX || !d_MX)
-    return QD_ERR_INVALID;
-  if (n == 0) return QD_OK;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (vec_fp32)
-    return launch<float>(n, width, b, ldx, ldy, d_rowptr, d_col, d_H, d_Himag, d_M, d_X, d_AX,
-                         d_MX, s);
-  return launch<double>(n, width, b, ldx, ldy, d_rowptr, d_col, d_H, d_Himag, d_M, d_X, d_AX, d_MX,
-                        s);
+  return qd_cap_spmm_pattern(n, 0, width, b, vec_fp32, d_rowptr, d_col, d_H, d_Himag, d_M, d_X, ldx,
+                             d_AX, d_MX, ldy, stream);
 }
 
 extern "C" int qd_cap_spmm(int32_t n, int b, int vec_fp32, const int32_t *d_rowptr,
                            const int32_t *d_col, const void *d_H, const void *d_Himag,
                            const void *d_M, const void *d_X, int ldx, void *d_AX, void *d_MX,
                            int ldy, void *stream) {
-  return qd_cap_spmm_lattice(n, 0, b, vec_fp32, d_rowptr, d_col, d_H, d_Himag, d_M, d_X, ldx, d_AX,
-                             d_MX, ldy, stream);
+  return qd_cap_spmm_pattern(n, 0, 0, b, vec_fp32, d_rowptr, d_col, d_H, d_Himag, d_M, d_X, ldx,
+                             d_AX, d_MX, ldy, stream);
 }

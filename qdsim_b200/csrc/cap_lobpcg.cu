@@ -1255,7 +1255,7 @@ size_t carve(qd::Arena &ar, int32_t n, int b, bool mixed, size_t dst_bytes, Work
 }
 
 struct Problem {
-  int32_t n;
+  int32_t n, nnz;
   const int32_t *rowptr, *col;
   const void *H, *G, *M;        // FP64
   const void *H32, *G32, *M32;  // FP32 copies (mixed form)
@@ -1284,8 +1284,8 @@ int lobpcg_run(const Problem &P, Work &w, Blocks &bl, int &cur, double tol, int 
   auto AS = [&](int i) { return static_cast<T2 *>(bl.AS[i]); };
   auto MS = [&](int i) { return static_cast<T2 *>(bl.MS[i]); };
   auto spmm = [&](int blk, int c0, int m) {
-    return qd_cap_spmm_lattice(n, P.prec ? P.prec->nx : 0, m, f32 ? 1 : 0, P.rowptr, P.col, H, G, M,
-                               S(blk) + c0, ld, AS(blk) + c0, MS(blk) + c0, ld, s);
+    return qd_cap_spmm_pattern(n, P.nnz, P.prec ? P.prec->nx : 0, m, f32 ? 1 : 0, P.rowptr, P.col, H,
+                               G, M, S(blk) + c0, ld, AS(blk) + c0, MS(blk) + c0, ld, s);
   };
   QD_CUDA_TRY(smem_opt_in<cap_gram_kernel<T>>(size_t(2) * kGStages * kGRows * kGT * sizeof(T2)));
   QD_CUDA_TRY(smem_opt_in<cap_chol_kernel>(kCholSmem));
@@ -1490,7 +1490,12 @@ extern "C" int qd_cap_lobpcg_solve(int32_t n, const int32_t *d_rowptr, const int
   Work w;
   const size_t need = carve(ar, n, b, mixed, dst, w);
   if (need > work_bytes || !w.res) return QD_ERR_WORKSPACE;
-  Problem P{n, d_rowptr, d_col, d_H, d_Himag, d_M, d_H32, d_Himag32, d_M32, h_prec, d_prec_mats,
+  // the products choose their kernel by the nonzeros per row
+  int32_t nnz = 0;
+  QD_CUDA_TRY(cudaMemcpyAsync(&nnz, d_rowptr + n, sizeof(nnz), cudaMemcpyDeviceToHost,
+                              static_cast<cudaStream_t>(stream)));
+  QD_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+  Problem P{n, nnz, d_rowptr, d_col, d_H, d_Himag, d_M, d_H32, d_Himag32, d_M32, h_prec, d_prec_mats,
             b, nev, eig_scale, static_cast<cudaStream_t>(stream)};
   cudaStream_t s = P.s;
   const int ld = 3 * b;
