@@ -115,3 +115,45 @@ def test_a_cap_that_is_enough_for_the_diagonal_form_only(cuda):
     prob, err = _solve(cuda, om, m, eps, 1, max_iter=18)
     assert prob._plan is not None and err <= 1e-9
     assert prob._least_cap(1e-12) > 18
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", [(60, 20), (7, 90)])
+@pytest.mark.parametrize("nrhs", [1, 3, 64])
+def test_diagonal_form_matches_the_oracle(cuda, nx, ny, nrhs):
+    """Contrast along y beyond the lattice form's bound."""
+    om, m = _mesh(nx, ny)
+    eps = np.where(np.repeat(np.arange(ny) % 3 == 1, 2 * nx), 300.0, 1.0)
+    prob, err = _solve(cuda, om, m, eps, nrhs)
+    assert prob._plan is None and prob.last_relres <= 1e-12
+    # residual 1e-12 of the right-hand side, amplified by at most the square root of
+    # the stiffness's condition number (< 400 sqrt(300))
+    assert err <= 7e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nrhs", [(60, 30, 1), (33, 64, 5), (120, 41, 64)])
+@pytest.mark.parametrize("contrast", [8.0, 30.0, -40.0])
+def test_lattice_form_over_its_range_of_contrasts(cuda, nx, ny, nrhs, contrast):
+    """eps at random over a factor of 8 and 30 in every element, and in layers along
+    y with a factor of 40; the iterations stay within the bound that the cap is
+    compared with."""
+    om, m = _mesh(nx, ny)
+    if contrast > 0.0:
+        eps = np.exp(np.random.default_rng(nx).uniform(0.0, np.log(contrast), om.num_elements))
+    else:
+        eps = np.repeat(np.where(np.arange(ny) < ny // 2, 1.0, -contrast), 2 * nx)
+    prob, err = _solve(cuda, om, m, eps, nrhs)
+    assert prob._plan is not None and 1.5 < prob._kappa <= 64.0
+    assert prob.last_iters <= prob._least_cap(1e-12) and prob.last_iters < 2 * nx
+    # as above, < 400 sqrt(40)
+    assert err <= 3e-9
+
+
+@pytest.mark.gpu
+def test_long_lines_split_their_columns(cuda):
+    """600 columns: a block sweeps 16 right-hand sides, and the last takes one."""
+    om, m = _mesh(600, 8)
+    eps = np.random.default_rng(6).uniform(10.0, 14.0, om.num_elements)
+    prob, err = _solve(cuda, om, m, eps, 33)
+    assert prob._plan is not None and prob.last_iters <= 14 and err <= 1e-9
