@@ -2,6 +2,7 @@
 
     python kernels_bench.py cap_spmm [--prec fp64|fp32] [--b 48] [--launches 10]
     python kernels_bench.py pcg [--iters 32]
+    python kernels_bench.py poisson [--nrhs 64] [--launches 10]
     python kernels_bench.py interp [--points 16777216] [--gradient] [--sorted]
     python kernels_bench.py adjoint [--launches 10]
     python kernels_bench.py sc [--iters 6]
@@ -12,6 +13,8 @@
 prints ms per launch and GB/s of algorithmic bytes.  ``pcg``: the Jacobi-PCG
 of the p-n junction's Poisson step (P1 300x100 cells, 30,401 nodes, 64
 right-hand sides) for a fixed number of iterations; prints ms per iteration.
+``poisson``: the same step as the loop solves it (separable preconditioner, to
+1e-12) with nrhs right-hand sides; prints ms per solve and iterations.
 ``interp``: ``qd_fe_interpolate`` of one nodal field of the P2 400x200-cell
 mesh on 200x100 nm at uniformly random points (values, optionally gradients
 and elements), in random order or sorted by cell (``--sorted``, the order of
@@ -72,6 +75,7 @@ def pcg(iters: int, dev):
     from qdsim_b200.workloads import c5_junction
     j = c5_junction(64)
     prob = PoissonProblem(j.mesh, j.eps_r, device=dev)
+    prob._plan = None                           # the diagonal form
     rng = np.random.default_rng(0)
     rho = 1.6e5 * rng.standard_normal((j.mesh.num_nodes, 64))
     out = {}
@@ -93,6 +97,26 @@ def pcg(iters: int, dev):
     return {"kernels": ["pcg_spmv_kernel", "pcg_axpy_kernel"], "nodes": n, "nnz": int(nnz),
             "nrhs": 64, "iterations": iters, "ms_per_iteration": ms,
             "algorithmic_bytes_per_iteration": int(alg), "GBps": alg / (ms * 1e-3) / 1e9}
+
+
+def poisson(nrhs: int, launches: int, dev):
+    from qdsim_b200.poisson import PoissonProblem
+    from qdsim_b200.workloads import c5_junction
+    j = c5_junction(64)
+    prob = PoissonProblem(j.mesh, j.eps_r, device=dev)
+    rng = np.random.default_rng(0)
+    rho = torch.from_numpy(1.6e5 * rng.standard_normal((j.mesh.num_nodes, nrhs))).to(dev)
+    vn = np.resize(np.asarray(j.biases), nrhs)
+    prob.solve(rho, 0.0, vn)                    # solve 0 (warm-up)
+    torch.cuda.synchronize()
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    for _ in range(launches):
+        prob.solve(rho, 0.0, vn)
+    e1.record()
+    torch.cuda.synchronize()
+    return {"kernels": "lat_*_kernel", "nodes": j.mesh.num_nodes, "nrhs": nrhs,
+            "iterations": prob.last_iters, "ms_per_solve": e0.elapsed_time(e1) / launches}
 
 
 def interp(points: int, gradient: bool, ordered: bool, launches: int, dev):
@@ -179,12 +203,13 @@ def cap_solve(prec: str, cells: int, dev):
 
 def main(argv=None):
     ap = argparse.ArgumentParser(description=__doc__.split("\n")[0])
-    ap.add_argument("case", choices=["cap_spmm", "pcg", "interp", "adjoint", "sc", "cap_solve"])
+    ap.add_argument("case", choices=["cap_spmm", "pcg", "poisson", "interp", "adjoint", "sc", "cap_solve"])
     ap.add_argument("--prec", default="fp64", choices=["fp64", "fp32", "mixed"])
     ap.add_argument("--cells", type=int, default=400)
     ap.add_argument("--b", type=int, default=48)
     ap.add_argument("--launches", type=int, default=10)
     ap.add_argument("--iters", type=int, default=32)
+    ap.add_argument("--nrhs", type=int, default=64)
     ap.add_argument("--points", type=int, default=1 << 24)
     ap.add_argument("--gradient", action="store_true")
     ap.add_argument("--sorted", action="store_true")
@@ -196,6 +221,8 @@ def main(argv=None):
         r = cap_spmm(a.prec, a.b, a.launches, dev)
     elif a.case == "pcg":
         r = pcg(a.iters, dev)
+    elif a.case == "poisson":
+        r = poisson(a.nrhs, a.launches, dev)
     elif a.case == "adjoint":
         r = adjoint(a.launches, dev)
     elif a.case == "sc":
