@@ -742,7 +742,8 @@ template <typename TV, int B> struct GramCfg {
   static constexpr int NT = NB * (NB + 1) / 2;            // upper-triangle 4x4 blocks
   static constexpr int NM = sizeof(TV) == 8 ? 1 : 2;
   static constexpr int NT2 = NM == 2 ? NT : 2 * NT;       // tasks
-  static constexpr int RG = (256 / NT2) > 16 ? 16 : ((256 / NT2) > 0 ? (256 / NT2) : 1);
+  static constexpr int RGMAX = NM == 2 ? 32 : 16;
+  static constexpr int RG = (256 / NT2) > RGMAX ? RGMAX : ((256 / NT2) > 0 ? (256 / NT2) : 1);
   static constexpr int THREADS = ((NT2 * RG + 31) / 32) * 32;
 };
 
@@ -941,6 +942,8 @@ gram_kernel(const Chunk *chunks, const DotState *st, const TV *X, const TV *W, c
   if (RG > 1) {
     double *red = reinterpret_cast<double *>(dsm);   // NT2 * NA doubles < one stage
     static_assert(NT2 * NA * sizeof(double) <= PP::BAR_OFF, "reduction slots");
+    // rows summed in FP32 before FP64 takes over: 2, 6, 16 (and 22) at B = 4, 8, 12 (16)
+    static_assert(sizeof(TV) == 8 || (PP::BLK / B + RG - 1) / RG <= B * B / 8, "FP32 partial sums");
     for (int g = 1; g < RG; ++g) {
       if (worker && rg == g) {
 #pragma unroll
