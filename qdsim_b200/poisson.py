@@ -118,6 +118,7 @@ class PoissonProblem:
         self.right = np.abs(x - mesh.Lx) < 1e-9 * mesh.Lx
         self.d_fixed = torch.from_numpy((self.left | self.right).astype(np.int32)).to(self.device)
         self._ws = None
+        self._pays = {}        # right-hand sides: lattice_pays
         self._plan = self._lattice_plan(eps_r_elem)
         self.last_iters = 0
         self.last_relres = 0.0
@@ -171,7 +172,10 @@ class PoissonProblem:
         if self._plan is not None and max_iter >= self._least_cap(tol):
             r = rho if isinstance(rho, torch.Tensor) else torch.from_numpy(np.asarray(rho, np.float64))
             r = r.to(self.device, torch.float64).reshape(n, -1).contiguous()
-            if r.shape[1] <= LATTICE_MAX_RHS and lattice_pays(self.mesh, self._kappa, r.shape[1]):
+            nrhs = r.shape[1]
+            if nrhs not in self._pays:
+                self._pays[nrhs] = nrhs <= LATTICE_MAX_RHS and lattice_pays(self.mesh, self._kappa, nrhs)
+            if self._pays[nrhs]:
                 return self._solve_lattice(r, V_p, V_n, tol, max_iter, x0)
             rho = r
         b = self.rhs(rho)
