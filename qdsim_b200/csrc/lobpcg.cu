@@ -77,11 +77,11 @@ constexpr double kJacobiRel64 = 2e-15;   // relative Jacobi threshold, FP64 phas
 constexpr double kJacobiRel32 = 1e-10;   // FP32 phase
 constexpr double kJacobiRelMx = 1e-12;   // the mixed form's finishing phase
 constexpr double kCholPivot32 = 1e-5;    // smallest Cholesky pivot of the scaled Gram (FP32 phase)
-// ... in the mixed form's finishing phase: a basis of condition number below
-// ~1e4 orthonormalised by Cholesky keeps its orthogonality to ~1e-12, well
-// inside the 1e-9 eigenvalue target; worse bases go to SVQB
-// (the plain FP64 form as well: its SVQB kept directions down to 1e-12)
-constexpr double kCholPivotMx = 1e-4;
+// ... in FP64 (the plain form and the mixed form's finishing phase).  A basis above
+// it is orthonormal to ~1e-12, which does not reach the levels: solved to 1e-14 they
+// are as accurate as with SVQB, which keeps directions down to 1e-12 (1e-15 of the
+// spectrum on pencils of 255 to 841 rows, either form); worse bases go to SVQB.
+constexpr double kCholPivot64 = 1e-4;
 #ifndef QD_SVQB_TAU64
 #define QD_SVQB_TAU64 1e-12
 #endif
@@ -1605,9 +1605,10 @@ __device__ __forceinline__ void tridiag_lowest_cta(Tile<TM> &A, double *Z, int l
 // chains of small dependent steps and the barriers between them (about seven
 // cycles per instruction and warp).  With the matrices in registers, the
 // congruence in place of two triangular products, and bisection without
-// divisions a launch takes 132 us at B = 16 (64 dots) and 97 us at B = 12 where
-// the form in shared memory took 377 and 201 us (499 us with SVQB in every step
-// of the plain FP64 form, which now takes it only when a pivot is small).
+// divisions a launch takes 120 to 132 us at B = 16 (64 dots) and 100 us at B = 12
+// where the form in shared memory took 377 and 201 us (499 us with SVQB in every
+// step of the plain FP64 form; either form takes it only when a pivot is small:
+// 1.2 ms at B = 16).
 template <int B>
 __global__ void __launch_bounds__(256)
 rr_kernel(DotState *st, const double *partial, const double *norms, double *theta,
@@ -1746,7 +1747,7 @@ rr_kernel(DotState *st, const double *partial, const double *norms, double *thet
   const int tx = tid & 15, ty = tid >> 4;
   bool chol = true;
   {
-    const double pivot_floor = s.phase == 0 ? kCholPivot32 : kCholPivotMx;
+    const double pivot_floor = s.phase == 0 ? kCholPivot32 : kCholPivot64;
     const int mu = has_p ? m : 2 * B;
     for (int i = 0; i < mu; ++i) chol = chol && sD[i] > 0.0;
     if (chol) {
