@@ -49,6 +49,16 @@ def lattice_fits(nx, ny):
     return 8 * ny * ny + 16 * nodes <= max(LATTICE_PLAN_BYTES, NODE_BYTES * nodes)
 
 
+def on_lattice(mesh):
+    """Whether the nodes of a P1 structured mesh lie on its uniform lattice (a mesh
+    whose nodes were moved, e.g. graded towards a contact, is structured too)."""
+    p = mesh.nodes.reshape(mesh.ny + 1, mesh.nx + 1, 2)
+    x = np.arange(mesh.nx + 1) * (mesh.Lx / mesh.nx)
+    y = np.arange(mesh.ny + 1) * (mesh.Ly / mesh.ny)
+    return (np.abs(p[:, :, 0] - x).max() <= 1e-9 * mesh.Lx
+            and np.abs(p[:, :, 1] - y[:, None]).max() <= 1e-9 * mesh.Ly)
+
+
 def lattice_pays(mesh, kappa, nrhs):
     """Whether the lattice form is the faster one, by the iterations that either
     needs to 1e-12 and what an iteration takes (microseconds on a B200).
@@ -125,10 +135,11 @@ class PoissonProblem:
 
     def _lattice_plan(self, eps):
         """Device plan of the separable preconditioner, or None where the
-        diagonal form is taken (unstructured mesh, eps varying too much along
+        diagonal form is taken (nodes not on a lattice, eps varying too much along
         y, a lattice beyond the kernel's limits or too narrow to pay)."""
         m = self.mesh
-        if not isinstance(m, StructuredMesh) or not lattice_fits(m.nx, m.ny):
+        if (not isinstance(m, StructuredMesh) or not lattice_fits(m.nx, m.ny)
+                or not on_lattice(m)):
             return None
         gx, gy, self._kappa = lattice_means(m, eps)
         # one right-hand side is where the diagonal form's iteration costs most

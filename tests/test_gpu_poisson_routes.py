@@ -157,3 +157,16 @@ def test_long_lines_split_their_columns(cuda):
     eps = np.random.default_rng(6).uniform(10.0, 14.0, om.num_elements)
     prob, err = _solve(cuda, om, m, eps, 33)
     assert prob._plan is not None and prob.last_iters <= 14 and err <= 1e-9
+
+
+@pytest.mark.gpu
+def test_moved_nodes_take_the_diagonal_form(cuda):
+    """The separable operator is that of equal cells: on a structured mesh whose nodes
+    were moved (columns graded towards a contact) it would be the wrong operator."""
+    om, m = _mesh(40, 20)
+    eps = np.random.default_rng(3).uniform(10.0, 14.0, om.num_elements)
+    for mesh in (om, m):
+        mesh.nodes[:, 0] = mesh.Lx * (mesh.nodes[:, 0] / mesh.Lx) ** 3
+    prob, err = _solve(cuda, om, m, eps, 2)
+    # as above, the condition number that much larger as the smallest cell is narrower
+    assert prob._plan is None and err <= 1e-9 * 40
